@@ -60,6 +60,35 @@ struct Stage1Plan {
   int nchunk, n_btile, n_items, grid;
   int ntile_cull;
   double max_turns;
+  // track groups (vb_track.cu): 1 = the call plans them
+  int track;
+  int trk_level, trk_steps, trk_gpp, trk_groups;   // largest pixel-block level, steps, groups per pair, groups
+  int trk_chunk_pix, trk_nchunk, trk_grid;
+};
+
+// Shape of one track group: mode < 0 = left to the per-term kernel, else
+// polynomial | log2(slots per sub-group) << 4 | pixel-block level << 8; centre,
+// frame and curve (b = gamma a + kappa a^2 in the frame) of each sub-group.
+struct TrackSub {
+  double uc[3];
+  float e[9], gamma, kappa, pad;
+};
+struct TrackPlan {
+  int mode, pad;
+  TrackSub sub[4];
+};
+// One block of 64, 256 or 1024 pixels: centre and sine of the cone's half-angle,
+// cone axis and its cosine.
+struct TrackNode {
+  float4 cen, axis;
+};
+struct TrackBuffers {
+  TrackNode* node[3] = {};
+  unsigned* rmax = nullptr;
+  TrackPlan* plan = nullptr;
+  int *off = nullptr, *left = nullptr, *list = nullptr, *direct = nullptr, *count = nullptr;
+  float4 *q0 = nullptr, *d1 = nullptr, *d2 = nullptr, *p1 = nullptr, *p2 = nullptr;
+  float* t2 = nullptr;
 };
 
 struct Stage1Buffers {       // slices of a workspace
@@ -69,7 +98,14 @@ struct Stage1Buffers {       // slices of a workspace
   double2* partial = nullptr;
   int* queue = nullptr;
   unsigned* err = nullptr;
+  TrackBuffers trk;
 };
+struct Carve;
+void track_plan(Stage1Plan* p, int items_per_cta);
+void track_carve(const Stage1Plan& p, Carve& c, Stage1Buffers& x, bool pixels);
+int track_prepare_pixels(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s);
+int track_group(const vb_baselines* bl, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s);
+int track_sum(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s);
 
 int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts* o, Stage1Plan* p);
 size_t stage1_carve(const Stage1Plan& p, void* ws, size_t cap, Stage1Buffers* b, bool pack_pixels);

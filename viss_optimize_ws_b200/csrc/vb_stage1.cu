@@ -32,27 +32,17 @@
 #include "vb_common.cuh"
 #include "vb_geom.cuh"
 #include "vb_internal.h"
+#include "vb_stage1.cuh"
 
 namespace vb {
 
 constexpr int S1_THREADS = 256;
-constexpr int kClsHid = 0, kClsVis = 1, kClsMix = 2;
 // Kernel-internal cull variant: tile-cone culling whose visible tiles still take
 // the per-pixel test (vb_stage1_opts.mask_visible_tiles).  A template value of
 // its own, so that the default tile-cone kernel carries no extra test.
 constexpr int kCullTileconeMV = 3;
 template <int CULL>
 __host__ __device__ constexpr bool is_tilecone() { return CULL == VB_CULL_TILECONE || CULL == kCullTileconeMV; }
-
-// F32X phase reduction: magic = 1.5 * 2^29 keeps every partial sum of the FMA
-// chain in [2^29, 2^30) (|u| + |v| + |w| < 2^28); the double's ulp is then
-// 2^-23 turns, so each FMA rounds to nearest on the 2^-23-turn grid the FP32
-// angle is built on, and the low 23 bits of the double are the turn fraction:
-// one LOP3 turns them into the exact float 2^23 + k.
-constexpr double kMagic = 805306368.0;              // 1.5 * 2^29
-constexpr float kTwoPiF = 6.28318530717958647692f;
-constexpr float kAngScale = 6.28318530717958647692f * 1.1920928955078125e-7f;  // fl(2pi) * 2^-23
-constexpr double kMaxUvwF32X = 67108864.0;         // 2^26: 3 * 2^26 < 2^28
 
 struct S1Args {
   const PixRec* __restrict__ px;   // stage-1 pixel records (interleaved, one per pixel)
@@ -70,6 +60,7 @@ struct S1Args {
   double2* partial;
   unsigned long long* counters;
   unsigned* err;
+  const int *list, *count;   // baselines left by the track groups: list[0, count[1]); count[0] factored groups
 };
 
 
@@ -135,27 +126,6 @@ __device__ __forceinline__ int tile_class_rt(const S1Args& a, const Baseline& b,
 
 // Loads half-baseline ih into registers (upstream: viss_recon_kernel.cuh:231-240,
 // ..._vissfast.cuh:476-497).
-
-// Per-endpoint threshold of the per-pixel occlusion test: the test
-// "fl(d * invn) < cosphi" (d the FP32 dot of pixel and endpoint, rounded as
-// occ_dot rounds it) holds exactly when d < t, t being the smallest float with
-// fl(t * invn) >= cosphi: fl(d * invn) does not decrease as d grows (invn > 0).
-// The masked path then compares d with t instead of multiplying first, with
-// the same masks (two multiplies fewer per masked term: 1217.7 -> 1206.1 ms on
-// the nside-1024 day, 9.66 -> 9.64 ms at nside 256).
-__device__ __noinline__ float occ_threshold(float invn, float c) {
-  if (c != c || invn != invn) return -INFINITY;                  // the test never fails
-  if (invn == 0.0f) return c > 0.0f ? INFINITY : -INFINITY;      // fl(d * 0) = 0 against c
-  if (isinf(invn)) return 0.0f;                                  // d * inf: fails exactly for d < 0
-  float t = c / invn;                                            // within a few ulps; fixed below
-  for (int k = 0; k < 16 && !(t * invn >= c); ++k) t = nextafterf(t, INFINITY);
-  for (int k = 0; k < 16; ++k) {
-    const float p = nextafterf(t, -INFINITY);
-    if (p * invn >= c) t = p; else break;
-  }
-  return t;
-}
-
 __device__ __forceinline__ void load_baseline(const S1Args& a, int ih, bool raw, Baseline& b) {
   b.active = ih < a.n_half;
   const int i = b.active ? half_to_full_pos(ih, a.nbl) : 0;
@@ -239,49 +209,10 @@ __device__ constexpr float imag_sign() {
   return (MODE == VB_PREC_FP32_FP64PH || MODE == VB_PREC_FP32_DSPH) ? -1.0f : 1.0f;
 }
 
-// --- bulk-copy staging --------------------------------------------------------
-// One thread copies a stage's records (a contiguous range of the interleaved
-// global array) into this CTA's own shared memory with cp.async.bulk, which
-// signals an mbarrier when the bytes have landed; the other buffer is filled
-// while the CTA computes on this one.  No cluster multicast: the source is
-// always this GPU's own memory and the destination this CTA's shared memory.
-// (Measured on one B200 against the cooperative loads it replaced, which
-// staged through registers between two barriers per stage: 1231 against 1248
-// ms on the nside-1024 day, 9.72 against 9.80 ms at nside 256.)
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void bulk_stage_issue(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-  // shared memory the threads read before the preceding barrier is written by
-  // the async proxy next: order the two proxies
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-// Waits for the phase `parity` of the barrier to complete, at most kBulkWaitTries
-// polls; a wait that runs out sets ERR_WAIT_TIMEOUT (the outputs of the call
-// are then not to be trusted) and returns.
-constexpr int kBulkWaitTries = 1 << 22;
-__device__ __forceinline__ void bulk_stage_wait(unsigned long long* bar, unsigned parity, unsigned* err) {
-  for (int i = 0; i < kBulkWaitTries; ++i) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    if (done) return;
-  }
-  atomicOr(err, ERR_WAIT_TIMEOUT);
-}
-
 // Register budget per thread: 80 for 3 resident CTAs of 256 threads; 120 for
 // 2 (measured: 120 beats the full 128 the 2-CTA budget allows by ~2 % on the
 // nside-256 workload, 112 and below lose more to the extra scheduling limits).
-template <int MODE, int BPT, int MINB, int CULL>
+template <int MODE, int BPT, int MINB, int CULL, bool LIST>
 __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PixRec* s_px = reinterpret_cast<PixRec*>(smem_raw);
@@ -316,23 +247,30 @@ __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
     }
   };
 
+  // LIST: the baselines left by the track groups, list[0, count[1])
+  int n_btile = a.n_btile, n_items = a.n_items;
+  if constexpr (LIST) {
+    n_btile = (a.count[1] + S1_THREADS * BPT - 1) / (S1_THREADS * BPT);
+    n_items = n_btile * a.nchunk;
+  }
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) s_item = atomicAdd(a.queue, 1);
     __syncthreads();
     const int item = s_item;
-    if (item >= a.n_items) break;
+    if (item >= n_items) break;
     // chunk-major order: the CTAs running at one time share a pixel chunk,
     // which then stays in L2 while they stage it
-    const int chunk = item / a.n_btile;
-    const int btile = item - chunk * a.n_btile;
+    const int chunk = item / n_btile;
+    const int btile = item - chunk * n_btile;
 
     // --- per-thread baselines -------------------------------------------------
     Baseline bl[BPT];
 #pragma unroll
     for (int k = 0; k < BPT; ++k) {
       Baseline& b = bl[k];
-      const int ih = btile * (S1_THREADS * BPT) + warp * (32 * BPT) + k * 32 + lane;
+      int ih = btile * (S1_THREADS * BPT) + warp * (32 * BPT) + k * 32 + lane;
+      if constexpr (LIST) ih = ih < a.count[1] ? a.list[ih] : a.n_half;
       load_baseline(a, ih, raw, b);
       const float uu = b.uf, vv = b.vf, ww = b.wf;
       if (MODE == VB_PREC_FP32_FP64PH && b.active &&
@@ -549,7 +487,8 @@ __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
     }
 #pragma unroll
     for (int k = 0; k < BPT; ++k) {
-      const int ih = btile * (S1_THREADS * BPT) + warp * (32 * BPT) + k * 32 + lane;
+      int ih = btile * (S1_THREADS * BPT) + warp * (32 * BPT) + k * 32 + lane;
+      if constexpr (LIST) ih = ih < a.count[1] ? a.list[ih] : a.n_half;
       if (ih < a.n_half)
         a.partial[(int64_t)chunk * a.n_half + ih] =
             make_double2(accR[k], (double)imag_sign<MODE>() * accI[k]);
@@ -565,23 +504,215 @@ __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
   if (a.counters && threadIdx.x < 4) atomicAdd(&a.counters[threadIdx.x], s_cnt[threadIdx.x]);
 }
 
-// V[ih] = sum over chunks of the partials, in chunk order (accumulate: V += that sum).
-__global__ void k_reduce_partials(const double2* __restrict__ partial, int nchunk, int n_half,
-                                  double* __restrict__ V, int accumulate) {
-  for (int ih = blockIdx.x * blockDim.x + threadIdx.x; ih < n_half; ih += gridDim.x * blockDim.x) {
-    double r = 0.0, im = 0.0;
-    for (int c = 0; c < nchunk; ++c) {
-      double2 p = partial[(int64_t)c * n_half + ih];
+// Term counters of a call whose sum is factored: the classes and the warps of
+// k_stage1 (the same baselines per warp, tiles and sub-tiles) without the sums,
+// so that the counters do not depend on which kernel summed a baseline.
+// Bound: issue.  A tile well away from every horizon of the warp's baselines has
+// one class for all of them: 32 tiles at a time, a lane each, are compared with
+// the bounding cone of the warp's endpoints (a margin of 1e-3 rad, far above
+// what the class tests round), and only the others are classified baseline by
+// baseline (nside-1024 day: 38 ms without that shortcut).
+constexpr int kCountTiles = 128;   // tiles per work item
+template <int BPT, int CULL>
+__global__ void __launch_bounds__(S1_THREADS) k_term_counts(const S1Args a, int ntile) {
+  const int lane = threadIdx.x & 31;
+  const int n_w = (a.n_half + 32 * BPT - 1) / (32 * BPT);
+  const int n_t = (ntile + kCountTiles - 1) / kCountTiles;
+  if (a.count[0] == 0) return;                // nothing is factored: k_stage1 counts
+  unsigned long long cnt[4] = {0, 0, 0, 0};   // sums over the lanes
+  for (int64_t it = (int64_t)blockIdx.x * (S1_THREADS / 32) + (threadIdx.x >> 5); it < (int64_t)n_w * n_t;
+       it += (int64_t)gridDim.x * (S1_THREADS / 32)) {
+    const int wt = (int)(it / n_t), tt = (int)(it - (int64_t)wt * n_t) * kCountTiles;
+    Baseline bl[BPT];
+    int nact = 0;
+    float sx = 0.f, sy = 0.f, sz = 0.f, cmin = 2.f, cmax = -2.f, dmin = 1.f;
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) {
+      Baseline& b = bl[k];
+      load_baseline(a, wt * 32 * BPT + k * 32 + lane, false, b);
+      nact += __popc(__ballot_sync(0xffffffffu, b.active));
+      if (!b.active) continue;
+      sx += b.ux1 + b.ux2; sy += b.uy1 + b.uy2; sz += b.uz1 + b.uz2;
+      cmin = fminf(cmin, fminf(b.c1, b.c2));
+      cmax = fmaxf(cmax, fmaxf(b.c1, b.c2));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sx += __shfl_xor_sync(0xffffffffu, sx, o);
+      sy += __shfl_xor_sync(0xffffffffu, sy, o);
+      sz += __shfl_xor_sync(0xffffffffu, sz, o);
+      cmin = fminf(cmin, __shfl_xor_sync(0xffffffffu, cmin, o));
+      cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+    }
+    const float inv = rsqrtf(sx * sx + sy * sy + sz * sz);
+    sx *= inv; sy *= inv; sz *= inv;
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) {
+      const Baseline& b = bl[k];
+      if (!b.active) continue;
+      const float d1 = b.ux1 * sx + b.uy1 * sy + b.uz1 * sz, d2 = b.ux2 * sx + b.uy2 * sy + b.uz2 * sz;
+      dmin = d1 < dmin ? d1 : (d1 >= dmin ? dmin : -2.f);   // a NaN opens the cone
+      dmin = d2 < dmin ? d2 : (d2 >= dmin ? dmin : -2.f);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dmin = fminf(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
+    // angles: endpoints within rho of the axis, horizons in [phi0, phi1] (away from the poles of the test)
+    const float rho = acosf(dmin) + 1e-3f, phi0 = acosf(cmax), phi1 = acosf(cmin);
+    const bool shortcut = dmin > 0.1f && cmin > -0.998f && cmax < 0.998f;
+    for (int tb = tt; tb < ntile && tb < tt + kCountTiles; tb += 32) {
+      const int mine = tb + lane;
+      bool open = mine < ntile;
+      if (open && shortcut) {
+        float D, A;
+        if constexpr (CULL == VB_CULL_EXACT) {
+          const ExactCone c = a.cones[mine];
+          D = acosf((float)c.cx * sx + (float)c.cy * sy + (float)c.cz * sz);
+          A = acosf((float)c.cos_a);
+        } else {
+          D = acosf(a.tcx[mine] * sx + a.tcy[mine] * sy + a.tcz[mine] * sz);
+          A = acosf(a.tcosA[mine]);
+        }
+        const int64_t t0 = (int64_t)mine * a.cull_tile;
+        const unsigned long long terms = (unsigned long long)nact * (unsigned long long)(min(a.npix, t0 + a.cull_tile) - t0);
+        if (D - rho - A >= phi1 + 1e-3f) {
+          cnt[2] += terms; cnt[3] += terms;
+          open = false;
+        } else if (CULL != kCullTileconeMV && D + rho + A <= phi0 - 1e-3f) {
+          cnt[0] += terms; cnt[3] += terms;
+          open = false;
+        }
+      }
+      unsigned todo = __ballot_sync(0xffffffffu, open);
+      while (todo) {
+        const int tile = tb + __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int64_t t0 = (int64_t)tile * a.cull_tile;
+        const int64_t t1 = min(a.npix, t0 + a.cull_tile);
+        bool any_live = false, any_mix = false;
+#pragma unroll
+        for (int k = 0; k < BPT; ++k) {
+          const int c = tile_class<CULL>(a, bl[k], tile);
+          bl[k].tcls = c;
+          any_live |= (c != kClsHid);
+          any_mix |= (c == kClsMix);
+        }
+        const bool live = __any_sync(0xffffffffu, any_live), mix = __any_sync(0xffffffffu, any_mix);
+        const unsigned long long terms = (unsigned long long)nact * (unsigned long long)(t1 - t0);
+        const bool refined = live && mix && is_tilecone<CULL>() && a.refine_pix > 0;
+        if (lane == 0) {
+          cnt[3] += terms;
+          if (!refined) cnt[!live ? 2 : (mix ? 1 : 0)] += terms;
+        }
+        if (!refined) continue;
+        bool l_vis = false;
+#pragma unroll
+        for (int k = 0; k < BPT; ++k) l_vis |= (bl[k].tcls == kClsVis);
+        const bool w_vis = __any_sync(0xffffffffu, l_vis);
+        const int nsub = (int)((t1 - t0 + a.refine_pix - 1) / a.refine_pix);
+        const int64_t sub0 = t0 / a.refine_pix;
+        for (int sb = 0; sb < nsub; sb += 32) {
+          bool sopen = sb + lane < nsub;
+          if (sopen && shortcut) {
+            const ExactCone c = a.subcones[sub0 + sb + lane];
+            const float D = acosf((float)c.cx * sx + (float)c.cy * sy + (float)c.cz * sz), A = acosf((float)c.cos_a);
+            const int64_t r0 = t0 + (int64_t)(sb + lane) * a.refine_pix;
+            const unsigned long long st = (unsigned long long)nact * (unsigned long long)(min(t1, r0 + a.refine_pix) - r0);
+            // the undecided baselines become hidden (the tile's visible ones stay) or visible
+            if (D - rho - A >= phi1 + 1e-3f) {
+              cnt[w_vis ? 0 : 2] += st;
+              sopen = false;
+            } else if (D + rho + A <= phi0 - 1e-3f) {
+              cnt[0] += st;
+              sopen = false;
+            }
+          }
+          unsigned subs = __ballot_sync(0xffffffffu, sopen);
+          while (subs) {
+            const int sub = sb + __ffs(subs) - 1;
+            subs &= subs - 1;
+            const int64_t r0 = t0 + (int64_t)sub * a.refine_pix;
+            const int64_t r1 = min(t1, r0 + a.refine_pix);
+            bool l_live = false, l_mix = false;
+#pragma unroll
+            for (int k = 0; k < BPT; ++k) {
+              const Baseline& b = bl[k];
+              int e = b.tcls;
+              if (e == kClsMix)
+                e = exact_tile_class(a.subcones + sub0 + sub, b.x1, b.y1, b.z1, b.i1, b.c1, b.x2, b.y2, b.z2, b.i2, b.c2);
+              l_live |= (e != kClsHid);
+              l_mix |= (e == kClsMix);
+            }
+            const bool w_live = __any_sync(0xffffffffu, l_live), w_mix = __any_sync(0xffffffffu, l_mix);
+            if (lane == 0) cnt[!w_live ? 2 : (w_mix ? 1 : 0)] += (unsigned long long)nact * (unsigned long long)(r1 - r0);
+          }
+        }
+      }
+    }
+  }
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cnt[k] += __shfl_xor_sync(0xffffffffu, cnt[k], o);
+    if (lane == 0 && cnt[k]) atomicAdd(&a.counters[k], cnt[k]);
+  }
+}
+
+// The same without culling: one class for every term.
+__global__ void k_term_counts_plain(unsigned long long* counters, int which, unsigned long long terms, const int* count) {
+  if (count[0] == 0) return;
+  atomicAdd(&counters[which], terms);
+  atomicAdd(&counters[3], terms);
+}
+
+template <int BPT>
+static int term_counts(const S1Args& a, const Stage1Plan& p, cudaStream_t s) {
+  const int64_t items = ceil_div(p.n_half, 32 * BPT) * ceil_div(p.ntile_cull, kCountTiles);
+  const int grid = (int)std::min<int64_t>(ceil_div(items, S1_THREADS / 32), (int64_t)sm_count() * 32);
+  if (p.cull == VB_CULL_EXACT) k_term_counts<BPT, VB_CULL_EXACT><<<grid, S1_THREADS, 0, s>>>(a, p.ntile_cull);
+  else if (p.mask_visible) k_term_counts<BPT, kCullTileconeMV><<<grid, S1_THREADS, 0, s>>>(a, p.ntile_cull);
+  else k_term_counts<BPT, VB_CULL_TILECONE><<<grid, S1_THREADS, 0, s>>>(a, p.ntile_cull);
+  VB_LAUNCH_CHECK();
+  return VB_OK;
+}
+
+// V[ih] = sum over chunks of the partials in a fixed order (accumulate: V += that
+// sum).  Baselines of a factored track group (plan, nullable) have trk_nchunk
+// partials.  32 baselines by kReduceRows chunk rows a CTA: a call with few
+// baselines has many chunks, and one thread walking them alone waits for each
+// load (12,288 pixels x 1,120 baselines: 48 chunks).
+constexpr int kReduceRows = 8;
+__global__ void __launch_bounds__(32 * kReduceRows)
+k_reduce_partials(const double2* __restrict__ partial, int nchunk, int n_half, double* __restrict__ V, int accumulate,
+                  const TrackPlan* __restrict__ plan, int nbl, int gpp, int trk_nchunk) {
+  __shared__ double2 s_sum[kReduceRows][32];
+  const int ih = blockIdx.x * 32 + threadIdx.x;
+  double r = 0.0, im = 0.0;
+  if (ih < n_half) {
+    int nc = nchunk;
+    if (plan) {
+      const int step = ih / nbl;
+      if (plan[(ih - step * nbl) * gpp + step / kTrackGroup].mode >= 0) nc = trk_nchunk;
+    }
+#pragma unroll 4
+    for (int c = threadIdx.y; c < nc; c += kReduceRows) {
+      const double2 p = partial[(int64_t)c * n_half + ih];
       r += p.x;
       im += p.y;
     }
-    if (accumulate) {
-      V[2 * ih] += r;
-      V[2 * ih + 1] += im;
-    } else {
-      V[2 * ih] = r;
-      V[2 * ih + 1] = im;
-    }
+  }
+  s_sum[threadIdx.y][threadIdx.x] = make_double2(r, im);
+  __syncthreads();
+  if (threadIdx.y != 0 || ih >= n_half) return;
+#pragma unroll
+  for (int k = 1; k < kReduceRows; ++k) {
+    r += s_sum[k][threadIdx.x].x;
+    im += s_sum[k][threadIdx.x].y;
+  }
+  if (accumulate) {
+    V[2 * ih] += r;
+    V[2 * ih + 1] += im;
+  } else {
+    V[2 * ih] = r;
+    V[2 * ih + 1] = im;
   }
 }
 
@@ -617,20 +748,22 @@ __global__ void k_phase_correct_expand(const double* __restrict__ Vr, const floa
 // ---------------------------------------------------------------------------
 // Kernel variants: precision x cull mode x baselines per thread x the
 // resident-CTA count the register budget is built for (3 CTAs/SM = 80
-// registers, only with BPT <= 2).
-template <int MODE, int CULL>
+// registers, only with BPT <= 2); for the FP32 sum with FP64 phase also over
+// the list of baselines that the track groups leave (a variant of its own: the
+// list in the plain kernel cost every other call 1 %, the smallest ones 5-8 %).
+template <int MODE, int CULL, bool LIST>
 static void* stage1_kernel(int bpt, int minb) {
-  if (bpt == 1) return minb == 3 ? (void*)k_stage1<MODE, 1, 3, CULL> : (void*)k_stage1<MODE, 1, 2, CULL>;
-  if (bpt == 2) return minb == 3 ? (void*)k_stage1<MODE, 2, 3, CULL> : (void*)k_stage1<MODE, 2, 2, CULL>;
-  return (void*)k_stage1<MODE, 4, 2, CULL>;
+  if (bpt == 1) return minb == 3 ? (void*)k_stage1<MODE, 1, 3, CULL, LIST> : (void*)k_stage1<MODE, 1, 2, CULL, LIST>;
+  if (bpt == 2) return minb == 3 ? (void*)k_stage1<MODE, 2, 3, CULL, LIST> : (void*)k_stage1<MODE, 2, 2, CULL, LIST>;
+  return (void*)k_stage1<MODE, 4, 2, CULL, LIST>;
 }
 
-template <int MODE>
+template <int MODE, bool LIST = false>
 static void* stage1_kernel_cull(int bpt, int minb, int cull) {
-  if (cull == VB_CULL_TILECONE) return stage1_kernel<MODE, VB_CULL_TILECONE>(bpt, minb);
-  if (cull == kCullTileconeMV) return stage1_kernel<MODE, kCullTileconeMV>(bpt, minb);
-  if (cull == VB_CULL_EXACT) return stage1_kernel<MODE, VB_CULL_EXACT>(bpt, minb);
-  return stage1_kernel<MODE, VB_CULL_NONE>(bpt, minb);
+  if (cull == VB_CULL_TILECONE) return stage1_kernel<MODE, VB_CULL_TILECONE, LIST>(bpt, minb);
+  if (cull == kCullTileconeMV) return stage1_kernel<MODE, kCullTileconeMV, LIST>(bpt, minb);
+  if (cull == VB_CULL_EXACT) return stage1_kernel<MODE, VB_CULL_EXACT, LIST>(bpt, minb);
+  return stage1_kernel<MODE, VB_CULL_NONE, LIST>(bpt, minb);
 }
 
 static void* stage1_kernel_of(int mode, int bpt, int minb, int cull) {
@@ -736,6 +869,7 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
   if (items > INT32_MAX) return fail(VB_ERR_UNSUPPORTED, "stage 1: too many work items");
   q.n_items = (int)items;
   if (q.grid > q.n_items) q.grid = q.n_items > 0 ? q.n_items : 1;
+  track_plan(&q, o->items_per_cta);
   *p = q;
   return VB_OK;
 }
@@ -749,8 +883,10 @@ size_t stage1_carve(const Stage1Plan& p, void* ws, size_t cap, Stage1Buffers* b,
     if (p.cull == VB_CULL_EXACT) x.cones = c.take<ExactCone>(p.ntile_cull);
     if (p.refine_pix > 0) x.subcones = c.take<ExactCone>((size_t)ceil_div(p.npix, p.refine_pix));
   }
-  x.partial = c.take<double2>((size_t)p.nchunk * (size_t)p.n_half);
+  const int rows = p.track ? std::max(p.nchunk, p.trk_nchunk) : p.nchunk;
+  x.partial = c.take<double2>((size_t)rows * (size_t)p.n_half);
   x.queue = c.take<int>(4);
+  track_carve(p, c, x, pack_pixels);
   if (b) *b = x;
   if (ws && !c.ok) return 0;
   return c.used();
@@ -760,7 +896,7 @@ int stage1_prepare_pixels(const vb_sky* sky, const Stage1Plan& p, const Stage1Bu
   VB_TRY(geom_pack_pixels(sky->B, sky->l, sky->m, sky->n, p.npix, b.px, s));
   if (p.cull == VB_CULL_EXACT) VB_TRY(geom_exact_cones(p.cull_tile, sky->l, sky->m, sky->n, p.npix, b.cones, s));
   if (p.refine_pix > 0) VB_TRY(geom_exact_cones(p.refine_pix, sky->l, sky->m, sky->n, p.npix, b.subcones, s));
-  return VB_OK;
+  return track_prepare_pixels(sky, p, b, s);
 }
 
 int stage1_run(const vb_sky* sky, const vb_baselines* bl, const Stage1Plan& p, const Stage1Buffers& b,
@@ -784,17 +920,45 @@ int stage1_run(const vb_sky* sky, const vb_baselines* bl, const Stage1Plan& p, c
   a.cp1 = bl->cosphi1; a.cp2 = bl->cosphi2; a.cosphi = bl->cosphi;
   a.n_half = p.n_half; a.nbl = p.nbl; a.blockage = p.blockage; a.phase_corrected = p.phase_corrected;
   a.queue = b.queue; a.partial = b.partial; a.counters = counters; a.err = b.err;
-  VB_CUDA(cudaMemsetAsync(b.queue, 0, sizeof(int), s));
-  size_t smem = 2 * (size_t)p.stage_pix * sizeof(PixRec);
-  const void* kern = stage1_kernel_of(p.precision, p.bpt, p.minb, p.mask_visible ? kCullTileconeMV : p.cull);
+  const int kcull = p.mask_visible ? kCullTileconeMV : p.cull;
+  const void* kern = stage1_kernel_of(p.precision, p.bpt, p.minb, kcull);
+  const size_t smem = 2 * (size_t)p.stage_pix * sizeof(PixRec);
   VB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  VB_CUDA(cudaMemsetAsync(b.queue, 0, 4 * sizeof(int), s));
+  if (p.track) {
+    // The device decides: with factored groups the plain kernel's queue starts
+    // past its last item and the list kernel runs, without any the other way
+    // round (three launches that end at once, about 10 us).
+    a.list = b.trk.direct;
+    a.count = b.trk.count;
+    VB_TRY(track_group(bl, p, b, s));
+    if (counters) {
+      if (p.cull == VB_CULL_NONE) {
+        k_term_counts_plain<<<1, 1, 0, s>>>(counters, p.blockage ? 1 : 0, (unsigned long long)p.n_half * p.npix,
+                                            b.trk.count);
+        VB_LAUNCH_CHECK();
+      } else {
+        VB_TRY(p.bpt == 1 ? term_counts<1>(a, p, s) : p.bpt == 2 ? term_counts<2>(a, p, s) : term_counts<4>(a, p, s));
+      }
+    }
+  }
   void* args[] = {&a};
   if (kbeg) VB_CUDA(record_event(kbeg, s));
+  if (p.track) {
+    VB_TRY(track_sum(sky, p, b, s));
+    S1Args la = a;
+    la.counters = nullptr;
+    la.queue = b.queue + 1;
+    const void* lk = stage1_kernel_cull<VB_PREC_FP32_FP64PH, true>(p.bpt, p.minb, kcull);
+    VB_CUDA(cudaFuncSetAttribute(lk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    void* largs[] = {&la};
+    VB_CUDA(cudaLaunchKernel(lk, dim3(p.grid), dim3(S1_THREADS), largs, smem, s));
+  }
   VB_CUDA(cudaLaunchKernel(kern, dim3(p.grid), dim3(S1_THREADS), args, smem, s));
   if (kend) VB_CUDA(record_event(kend, s));
-  int rg = (int)ceil_div(p.n_half, 256);
-  if (rg > sm_count() * 16) rg = sm_count() * 16;
-  k_reduce_partials<<<rg, 256, 0, s>>>(b.partial, p.nchunk, p.n_half, V_half, accumulate ? 1 : 0);
+  k_reduce_partials<<<(int)ceil_div(p.n_half, 32), dim3(32, kReduceRows), 0, s>>>(b.partial, p.nchunk, p.n_half, V_half,
+                                                                                 accumulate ? 1 : 0,
+                                                                                 p.track ? b.trk.plan : nullptr, p.nbl, p.trk_gpp, p.trk_nchunk);
   VB_LAUNCH_CHECK();
   return VB_OK;
 }
@@ -831,6 +995,10 @@ extern "C" int vb_viss_halfsym(const vb_sky* sky, const vb_baselines* bl, const 
     return fail(VB_ERR_INVALID, "vb_viss_halfsym: endpoint arrays missing");
   Stage1Buffers b;
   size_t need = stage1_carve(p, nullptr, 0, nullptr, true);
+  if (p.track && ws_bytes < need) {   // the per-term kernel alone needs less
+    p.track = 0;
+    need = stage1_carve(p, nullptr, 0, nullptr, true);
+  }
   if (!workspace || ws_bytes < need)
     return fail(VB_ERR_NOMEM, "vb_viss_halfsym: workspace %zu bytes < %zu", ws_bytes, need);
   if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
@@ -882,6 +1050,7 @@ extern "C" int vb_stage1_tile_classes(const vb_sky* sky, const vb_baselines* bl,
     }
   }
   Stage1Buffers b;
+  p.track = 0;
   size_t need = stage1_carve(p, nullptr, 0, nullptr, true);
   if (!workspace || ws_bytes < need)
     return fail(VB_ERR_NOMEM, "vb_stage1_tile_classes: workspace %zu bytes < %zu", ws_bytes, need);
