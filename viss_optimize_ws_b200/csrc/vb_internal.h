@@ -128,11 +128,32 @@ struct Stage2Plan {
   int nblocks;          // pixel blocks
   int nchunk_target;    // group chunks per pixel block (upper bound; sizes the partials)
   size_t cub_sort_bytes, cub_scan_bytes;
+  // clusters of groups (vb_track2.cu): 1 = the call plans them
+  int trk, trk_ntrk, trk_entries, trk_blocks, trk_rows;
 };
+struct GroupCluster;
+struct GroupRec;
+struct ClusterBuffers {
+  int *count = nullptr, *slots = nullptr, *order = nullptr, *dst = nullptr, *list = nullptr;
+  GroupCluster *table = nullptr, *clu = nullptr;
+  vb_seg_params* spd = nullptr;
+  unsigned* rmax = nullptr;
+  TrackNode* node[3] = {};
+};
+void cluster_plan(Stage2Plan* p, int nbl);
+void cluster_carve(const Stage2Plan& p, Carve& c, ClusterBuffers& x);
+int cluster_group(const Stage2Plan& p, const ClusterBuffers& x, const unsigned long long* skeys,
+                  const int* svals, const int* start, const int* ngroups, const vb_seg_params* sp, const int* seg_t0,
+                  const int* seg_tlen, cudaStream_t s);
+int cluster_sum(const vb_sky* sky, const Stage2Plan& p, const ClusterBuffers& x, const vb_seg_params* sp, const GroupRec* rec,
+                const int* ngroups, int* queue, double* Cpart, unsigned* Wpart, cudaStream_t s);
+// Pixel-block nodes and radii of a sky (vb_track.cu); B may be NULL.
+int track_nodes(const float* B, const float* l, const float* m, const float* n, int64_t npix, TrackNode* const (&node)[3],
+                unsigned* rmax, cudaStream_t s);
 struct Stage2Pixels {       // per-pixel state the caller already prepared
   bool cones_ready = false;  // block cones already computed in this workspace
 };
-int stage2_plan(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* o, Stage2Plan* p);
+int stage2_plan(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* o, Stage2Plan* p, int nbl);
 // Exact cones of the stage-2 pixel blocks into the workspace (VB_CULL_EXACT);
 // stage2_run then skips them when Stage2Pixels::cones_ready is set.
 int stage2_prepare_cones(const vb_sky* sky, const Stage2Plan& p, void* ws, size_t cap, cudaStream_t st);
@@ -144,8 +165,8 @@ struct Stage2Groups {
   int sorted_keys_alt = 0;   // the sorted keys / indices sit in the second buffer of their pair
   int sorted_vals_alt = 0;
 };
-int stage2_group(const vb_baselines* bl, int nseg, const int* seg_t0, const int* seg_tlen, const Stage2Plan& p,
-                 void* ws, size_t cap, cudaStream_t s, Stage2Groups* out);
+int stage2_group(const vb_sky* sky, const vb_baselines* bl, int nseg, const int* seg_t0, const int* seg_tlen,
+                 const Stage2Plan& p, void* ws, size_t cap, cudaStream_t s, Stage2Groups* out, const Stage2Pixels* pre);
 int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half, int nseg, const Stage2Plan& p,
                   void* ws, size_t cap, const Stage2Groups& gr, float* C, uint32_t* W, vb_seg_params* seg_params,
                   unsigned long long* counters, double* w_scalar_total, cudaStream_t s, const Stage2Pixels* pre,

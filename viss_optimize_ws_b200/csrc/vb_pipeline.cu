@@ -548,7 +548,9 @@ static int enqueue_stages(vb_pipeline* p) {
   Stage2Groups gr;
   // the side stream is joined back on every path, so that a failed step never
   // leaves it forked from a stream capture
-  int rc = stage2_group(&bl, p->nseg, p->d_t0, p->d_tlen, p->p2, p->ws2, p->ws2_bytes, p->s_side, &gr);
+  Stage2Pixels pre;
+  pre.cones_ready = p->s2_cones_ready;
+  int rc = stage2_group(&sky, &bl, p->nseg, p->d_t0, p->d_tlen, p->p2, p->ws2, p->ws2_bytes, p->s_side, &gr, &pre);
   const cudaError_t ej = cudaEventRecord(p->join, p->s_side);
   if (rc == VB_OK)
     rc = stage1_run(&sky, &bl, p->p1, p->b1, true, p->Vd, p->counters, p->s, p->ev[5], p->ev[6]);
@@ -560,8 +562,6 @@ static int enqueue_stages(vb_pipeline* p) {
   const cudaError_t ew = (ej == cudaSuccess) ? cudaStreamWaitEvent(p->s, p->join, 0) : ej;
   if (rc != VB_OK) return rc;
   VB_CUDA(ew);
-  Stage2Pixels pre;
-  pre.cones_ready = p->s2_cones_ready;
   VB_TRY(stage2_finish(&sky, &bl, p->Vh, p->nseg, p->p2, p->ws2, p->ws2_bytes, gr, p->C, p->W, p->segp,
                        p->counters + 4, p->wsum, p->s, &pre, p->ev[7], p->ev[8]));
   VB_CUDA(record_event(p->ev[2], p->s));
@@ -608,7 +608,7 @@ static int plan_stages(vb_pipeline* p) {
   o2.bl_max = effective_bl_max(p);
   o2.lambda = c->lambda_m;
   Stage2Plan p2;
-  VB_TRY(stage2_plan(p->n_half, p->nseg, p->nres, &o2, &p2));
+  VB_TRY(stage2_plan(p->n_half, p->nseg, p->nres, &o2, &p2, p->nbl));
   drop_graph(p);
   if (p->s) VB_CUDA(cudaStreamSynchronize(p->s));
   VB_TRY(regrow(p, &p->ws1, &p->ws1_bytes, stage1_carve(p1, nullptr, 0, nullptr, true)));
@@ -800,7 +800,8 @@ static int run_slabs(vb_pipeline* p, const float* B_host, int scale, float* C_ho
     vb_sky sky = sky_of(p);
     sky.npix = cnt;
     Stage2Plan q{};
-    VB_TRY(stage2_plan(p->n_half, p->nseg, cnt, &o2, &q));
+    VB_TRY(stage2_plan(p->n_half, p->nseg, cnt, &o2, &q, p->nbl));
+    if (q.trk && stage2_workspace(q, nullptr, 0, nullptr) > p->ws2_bytes) q.trk = 0;
     VB_TRY(stage2_run(&sky, &bl, p->Vh, p->nseg, p->d_t0, p->d_tlen, q, p->ws2, p->ws2_bytes, p->C, p->W, p->segp,
                       p->counters + 4, p->wsum, p->s, nullptr));
     VB_CUDA(cudaMemcpyAsync(C_host + base, p->C, cnt * sizeof(float), cudaMemcpyDeviceToHost, p->s));

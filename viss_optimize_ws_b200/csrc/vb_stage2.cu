@@ -18,12 +18,14 @@
 //  finalize: C = sum C / sum W (blockage=1) or C / sum nuniq (blockage=0).
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 
 #include "vb_common.cuh"
 #include "vb_geom.cuh"
 #include "vb_internal.h"
+#include "vb_stage2.cuh"
 
 namespace vb {
 
@@ -33,16 +35,6 @@ constexpr double kMagic2 = 805306368.0;  // 1.5 * 2^29: 2^-23-turn ulp, see stag
 constexpr float kTwoPiF2 = 6.28318530717958647692f;
 constexpr float kAngScale2 = 6.28318530717958647692f * 1.1920928955078125e-7f;
 
-struct GroupRec {         // 96 bytes
-  double a, b, c;         // t = a l + b m + c n  (a = ugu, b = vgu, c = ugu fa + vgu fb)
-  float vx, vy;           // representative / averaged visibility
-  float fa, fb;
-  float cp1, cp2;         // horizon cosines of the representative endpoints
-  float4 p1, p2;          // (x, y, z, invn) of the representative endpoints
-  float chi, clo;         // c split into two floats (double-single phase)
-  int key, flags;         // flags: bit0 = skip (key 0 / nothing to add), bit1 = non-finite V,
-                          // bits 2.. = segment
-};
 struct GroupMeta {        // members of a group (member-sampling path)
   int s0, L, seg, pad;
 };
@@ -91,16 +83,23 @@ __device__ __forceinline__ float dd_to_float(dd a) {
 }
 
 // --- per-segment fit ---------------------------------------------------------
-__global__ void __launch_bounds__(256) k_seg_fit(const float* __restrict__ u, const float* __restrict__ v,
+// One CTA per segment.  Latency of its own loads: 1024 threads (a segment of
+// 112,000 baselines: 300 us with 256).
+constexpr int kFitThreads = 1024;
+__device__ __forceinline__ dd dd_shfl_xor(dd a, int m) {
+  return {__shfl_xor_sync(0xffffffffu, a.hi, m), __shfl_xor_sync(0xffffffffu, a.lo, m)};
+}
+__global__ void __launch_bounds__(kFitThreads) k_seg_fit(const float* __restrict__ u, const float* __restrict__ v,
                                                  const float* __restrict__ w, int nbl, const int* __restrict__ seg_t0,
                                                  const int* __restrict__ seg_tlen, float bl_max, float lambda,
                                                  int grid_res, int mirror, vb_seg_params* __restrict__ out) {
-  __shared__ dd red[5][256];
+  __shared__ dd red[5][kFitThreads / 32];
   const int s = blockIdx.x;
   const int i0 = 2 * nbl * seg_t0[s];
   const int n = 2 * nbl * seg_tlen[s];
   dd a[5];
   for (int k = 0; k < 5; ++k) a[k] = {0.0, 0.0};
+#pragma unroll 2
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     double uu = u[i0 + i], vv = v[i0 + i], ww = w[i0 + i];
     a[0] = dd_add(a[0], dd_from_prod(uu, uu));
@@ -109,13 +108,18 @@ __global__ void __launch_bounds__(256) k_seg_fit(const float* __restrict__ u, co
     a[3] = dd_add(a[3], dd_from_prod(uu, ww));
     a[4] = dd_add(a[4], dd_from_prod(vv, ww));
   }
-  for (int k = 0; k < 5; ++k) red[k][threadIdx.x] = a[k];
-  __syncthreads();
-  for (int off = 128; off > 0; off >>= 1) {
-    if (threadIdx.x < off)
-      for (int k = 0; k < 5; ++k) red[k][threadIdx.x] = dd_add(red[k][threadIdx.x], red[k][threadIdx.x + off]);
-    __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int k = 0; k < 5; ++k) {
+    for (int off = 16; off > 0; off >>= 1) a[k] = dd_add(a[k], dd_shfl_xor(a[k], off));
+    if (lane == 0) red[k][warp] = a[k];
   }
+  __syncthreads();
+  if (warp == 0)
+    for (int k = 0; k < 5; ++k) {
+      dd x = red[k][lane];
+      for (int off = 16; off > 0; off >>= 1) x = dd_add(x, dd_shfl_xor(x, off));
+      if (lane == 0) red[k][0] = x;
+    }
   if (threadIdx.x != 0) return;
   dd su2 = red[0][0], sv2 = red[1][0], suv = red[2][0], suw = red[3][0], svw = red[4][0];
   dd p = dd_mul(su2, sv2);
@@ -229,6 +233,7 @@ struct RecArgs {
   GroupRec* rec;
   GroupMeta* meta;
   unsigned* err;
+  const int* dst;       // nullable: place of each group's record (clusters in use)
 };
 
 __global__ void k_group_records(const RecArgs r, int max_groups) {
@@ -286,7 +291,7 @@ __global__ void k_group_records(const RecArgs r, int max_groups) {
       // full-grid path tests finiteness of V before use (viss_recon_kernel.cuh:595)
       if (!r.mirror && !(isfinite(o.vx) && isfinite(o.vy))) o.flags |= 2;
     }
-    r.rec[g] = o;
+    r.rec[r.dst ? r.dst[g] : g] = o;
     if (r.meta) r.meta[g] = GroupMeta{s0, L, seg, 0};
   }
 }
@@ -865,18 +870,27 @@ __global__ void __launch_bounds__(S2_THREADS) k_recon_members(const ReconArgs a)
   }
 }
 
+// clusters (nullable): {clusters, groups of the per-term partials}; the
+// clusters' partials are trk_rows rows after the nchunk_target ones.
 __global__ void k_finalize(const double* __restrict__ Cpart, const unsigned* __restrict__ Wpart,
                            const int* __restrict__ ngroups, int nchunk_target, int64_t npix, int blockage,
-                           float* __restrict__ C, uint32_t* __restrict__ W, double* __restrict__ wsum_out) {
+                           float* __restrict__ C, uint32_t* __restrict__ W, double* __restrict__ wsum_out,
+                           const int* __restrict__ clusters, int trk_rows) {
   const int ng = *ngroups;
-  const int gchunk = group_chunk(ng, nchunk_target);
-  const int nchunk = (ng + gchunk - 1) / gchunk;
+  const int nrec = clusters ? clusters[1] : ng;
+  const int gchunk = group_chunk(nrec, nchunk_target);
+  const int nchunk = (nrec + gchunk - 1) / gchunk;
+  const int row1 = clusters && clusters[0] > 0 ? nchunk_target + trk_rows : nchunk_target;
   if (blockIdx.x == 0 && threadIdx.x == 0 && wsum_out) *wsum_out = (double)ng;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < npix; p += stride) {
     double c = 0.0;
     unsigned w = 0;
     for (int k = 0; k < nchunk; ++k) {
+      c += Cpart[(int64_t)k * npix + p];
+      w += Wpart[(int64_t)k * npix + p];
+    }
+    for (int k = nchunk_target; k < row1; ++k) {
       c += Cpart[(int64_t)k * npix + p];
       w += Wpart[(int64_t)k * npix + p];
     }
@@ -888,8 +902,38 @@ __global__ void k_finalize(const double* __restrict__ Cpart, const unsigned* __r
   }
 }
 
+// Term counters of the groups that the clusters sum: the classes that
+// k_recon_rec would give them against its pixel blocks, a warp per block and 32
+// groups, so that the counters do not depend on which kernel summed a group.
+__global__ void k_cluster_counts(const ReconArgs a, const int* count, const int* ngroups) {
+  const int lane = threadIdx.x & 31;
+  const int nd = count[1], n = *ngroups - nd;
+  if (count[0] == 0 || n <= 0) return;
+  const int per = (n + 31) / 32;
+  unsigned long long cnt[4] = {0, 0, 0, 0};
+  for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < (int64_t)per * a.nblocks;
+       it += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int blk = (int)(it / per), g = (int)(it - (int64_t)blk * per) * 32 + lane;
+    if (g >= n) continue;
+    const GroupRec* r = a.rec + nd + g;
+    const unsigned long long npx = (unsigned long long)min((int64_t)a.block_pix, a.npix - (int64_t)blk * a.block_pix);
+    int cls = 0;
+    if (!(r->flags & 3)) {
+      if (!a.blockage) cls = 1;
+      else if (a.cull == VB_CULL_EXACT) cls = exact_group_class(a.cones + blk, r->p1, r->cp1, r->p2, r->cp2);
+      else cls = 2;
+    }
+    cnt[cls == 1 ? 0 : (cls == 2 ? 1 : 2)] += npx;
+    cnt[3] += npx;
+  }
+  for (int k = 0; k < 4; ++k) {
+    for (int o = 16; o > 0; o >>= 1) cnt[k] += __shfl_xor_sync(0xffffffffu, cnt[k], o);
+    if (lane == 0 && cnt[k]) atomicAdd(&a.counters[k], cnt[k]);
+  }
+}
+
 // ---------------------------------------------------------------------------
-int stage2_plan(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* o, Stage2Plan* p) {
+int stage2_plan(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* o, Stage2Plan* p, int nbl) {
   if (!o || !p) return fail(VB_ERR_INVALID, "stage 2: null argument");
   if (n_half_total < 0 || nseg <= 0 || npix <= 0)
     return fail(VB_ERR_INVALID, "stage 2: n_half_total=%d nseg=%d npix=%lld", n_half_total, nseg, (long long)npix);
@@ -943,6 +987,7 @@ int stage2_plan(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* 
     return fail(VB_ERR_CUDA, "stage 2: CUB scan size query failed");
   q.cub_sort_bytes = sort_bytes;
   q.cub_scan_bytes = scan_bytes;
+  cluster_plan(&q, nbl);
   *p = q;
   return VB_OK;
 }
@@ -961,6 +1006,7 @@ struct S2Slices {
   void* cub_sort;
   void* cub_scan;
   double* wsum;
+  ClusterBuffers trk;
 };
 
 static size_t carve2(const Stage2Plan& p, void* ws, size_t cap, S2Slices* s) {
@@ -981,21 +1027,25 @@ static size_t carve2(const Stage2Plan& p, void* ws, size_t cap, S2Slices* s) {
   x.wsum = c.take<double>(2);
   x.rec = c.take<GroupRec>(n);
   x.meta = c.take<GroupMeta>(n);
-  x.Cpart = c.take<double>((size_t)p.nchunk_target * (size_t)p.npix);
-  x.Wpart = c.take<unsigned>((size_t)p.nchunk_target * (size_t)p.npix);
+  const size_t rows = (size_t)p.nchunk_target + (p.trk ? p.trk_rows : 0);
+  x.Cpart = c.take<double>(rows * (size_t)p.npix);
+  x.Wpart = c.take<unsigned>(rows * (size_t)p.npix);
   x.cones = c.take<ExactCone>(p.nblocks);
   x.Vfull = p.mirror ? nullptr : c.take<float>((size_t)4 * (p.n_half_total > 0 ? p.n_half_total : 1));
   x.cub_sort = c.take<char>(p.cub_sort_bytes);
   x.cub_scan = c.take<char>(p.cub_scan_bytes);
+  cluster_carve(p, c, x.trk);
   if (s) *s = x;
   if (ws && !c.ok) return 0;
   return c.used();
 }
 
 int stage2_prepare_cones(const vb_sky* sky, const Stage2Plan& p, void* ws, size_t cap, cudaStream_t st) {
-  if (p.cull != VB_CULL_EXACT) return VB_OK;
+  if (p.cull != VB_CULL_EXACT && !p.trk) return VB_OK;
   S2Slices x;
   if (!carve2(p, ws, cap, &x)) return fail(VB_ERR_NOMEM, "stage 2: workspace too small (%zu bytes)", cap);
+  if (p.trk) VB_TRY(track_nodes(nullptr, sky->l, sky->m, sky->n, p.npix, x.trk.node, x.trk.rmax, st));
+  if (p.cull != VB_CULL_EXACT) return VB_OK;
   return geom_exact_cones(p.block_pix, sky->l, sky->m, sky->n, p.npix, x.cones, st);
 }
 
@@ -1040,8 +1090,8 @@ __global__ void k_expand_half(const float* __restrict__ Vh, int n_half, int nbl,
 // Steps 1-4 read only the baselines (u, v and the segment table), so a caller
 // may run them on a second stream concurrently with stage 1; the sort's
 // double-buffer choice is known at enqueue time and handed to stage2_finish.
-int stage2_group(const vb_baselines* bl, int nseg, const int* seg_t0, const int* seg_tlen, const Stage2Plan& p,
-                 void* ws, size_t cap, cudaStream_t st, Stage2Groups* out) {
+int stage2_group(const vb_sky* sky, const vb_baselines* bl, int nseg, const int* seg_t0, const int* seg_tlen,
+                 const Stage2Plan& p, void* ws, size_t cap, cudaStream_t st, Stage2Groups* out, const Stage2Pixels* pre) {
   S2Slices x;
   if (!carve2(p, ws, cap, &x)) return fail(VB_ERR_NOMEM, "stage 2: workspace too small (%zu bytes)", cap);
   const int n = p.n_keyed_total;
@@ -1054,7 +1104,7 @@ int stage2_group(const vb_baselines* bl, int nseg, const int* seg_t0, const int*
   int g = (int)ceil_div(n > 0 ? n : 1, 256);
   if (g > sm_count() * 16) g = sm_count() * 16;
   // 1. per-segment fit
-  k_seg_fit<<<nseg, 256, 0, st>>>(bl->u, bl->v, bl->w, nbl, seg_t0, seg_tlen, p.bl_max, p.lambda, p.grid_res,
+  k_seg_fit<<<nseg, kFitThreads, 0, st>>>(bl->u, bl->v, bl->w, nbl, seg_t0, seg_tlen, p.bl_max, p.lambda, p.grid_res,
                                   p.mirror, x.sp);
   VB_LAUNCH_CHECK();
   if (n > 0) {
@@ -1078,6 +1128,11 @@ int stage2_group(const vb_baselines* bl, int nseg, const int* seg_t0, const int*
     VB_CUDA(cub::DeviceScan::InclusiveSum(x.cub_scan, scb, x.flags, x.gid, n, st));
     k_group_starts<<<g, 256, 0, st>>>(x.flags, x.gid, n, sk, x.start, x.ngroups, x.sp);
     VB_LAUNCH_CHECK();
+    // clusters of groups along the tracks (they need the blocks' radii)
+    if (p.trk) {
+      if (!(pre && pre->cones_ready)) VB_TRY(track_nodes(nullptr, sky->l, sky->m, sky->n, p.npix, x.trk.node, x.trk.rmax, st));
+      VB_TRY(cluster_group(p, x.trk, sk, dv.Current(), x.start, x.ngroups, x.sp, seg_t0, seg_tlen, st));
+    }
   }
   return VB_OK;
 }
@@ -1111,7 +1166,8 @@ int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half
     r.x2 = bl->x2; r.y2 = bl->y2; r.z2 = bl->z2; r.in2 = bl->invn2;
     r.cp1 = bl->cosphi1; r.cp2 = bl->cosphi2; r.cosphi = bl->cosphi;
     r.nbl = nbl; r.mirror = p.mirror; r.blockage = p.blockage; r.occ_mode = p.occ_mode;
-    r.rec = x.rec; r.meta = x.meta; r.err = x.err;
+    r.rec = x.rec; r.meta = p.trk ? nullptr : x.meta; r.err = x.err;
+    r.dst = p.trk ? x.trk.dst : nullptr;
     k_group_records<<<g, 256, 0, st>>>(r, n);
     VB_LAUNCH_CHECK();
   }
@@ -1132,8 +1188,21 @@ int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half
     ra.cones = x.cones; ra.queue = x.queue; ra.Cpart = x.Cpart; ra.Wpart = x.Wpart;
     ra.counters = counters; ra.err = x.err;
     const bool members = p.blockage && p.occ_mode != 2;
-    VB_CUDA(cudaMemsetAsync(x.queue, 0, sizeof(int), st));
+    VB_CUDA(cudaMemsetAsync(x.queue, 0, 2 * sizeof(int), st));
+    if (p.trk) {
+      // k_recon_rec sums the groups outside the clusters: their records come
+      // first, with segment ranges of their own
+      ra.ngroups = x.trk.count + 1;
+      ra.sp = x.trk.spd;
+      if (counters) {
+        k_cluster_counts<<<sm_count() * 8, 256, 0, st>>>(ra, x.trk.count, x.ngroups);
+        VB_LAUNCH_CHECK();
+      }
+    }
     if (kbeg) VB_CUDA(record_event(kbeg, st));
+    if (p.trk)
+      VB_TRY(cluster_sum(sky, p, x.trk, x.sp, x.rec, x.ngroups, x.queue + 1, x.Cpart + (size_t)p.nchunk_target * (size_t)p.npix,
+                         x.Wpart + (size_t)p.nchunk_target * (size_t)p.npix, st));
     switch (p.precision) {
       case VB_PREC_REF32: VB_TRY(launch_recon<VB_PREC_REF32>(ra, members, p.ppt, st)); break;
       case VB_PREC_FP64: VB_TRY(launch_recon<VB_PREC_FP64>(ra, members, p.ppt, st)); break;
@@ -1148,7 +1217,8 @@ int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half
   // 9. finalize: sum the group-chunk partials, normalise
   int gf = (int)ceil_div(p.npix, 256);
   if (gf > sm_count() * 16) gf = sm_count() * 16;
-  k_finalize<<<gf, 256, 0, st>>>(x.Cpart, x.Wpart, x.ngroups, p.nchunk_target, p.npix, p.blockage, C, W, x.wsum);
+  k_finalize<<<gf, 256, 0, st>>>(x.Cpart, x.Wpart, x.ngroups, p.nchunk_target, p.npix, p.blockage, C, W, x.wsum,
+                               p.trk && n > 0 ? x.trk.count : nullptr, p.trk_rows);
   VB_LAUNCH_CHECK();
   if (seg_params_out)
     VB_CUDA(cudaMemcpyAsync(seg_params_out, x.sp, nseg * sizeof(vb_seg_params), cudaMemcpyDeviceToDevice, st));
@@ -1161,7 +1231,7 @@ int stage2_run(const vb_sky* sky, const vb_baselines* bl, const float* V_half, i
                vb_seg_params* seg_params_out, unsigned long long* counters, double* w_scalar_total, cudaStream_t st,
                const Stage2Pixels* pre, cudaEvent_t kbeg, cudaEvent_t kend) {
   Stage2Groups gr;
-  VB_TRY(stage2_group(bl, nseg, seg_t0, seg_tlen, p, ws, cap, st, &gr));
+  VB_TRY(stage2_group(sky, bl, nseg, seg_t0, seg_tlen, p, ws, cap, st, &gr, pre));
   return stage2_finish(sky, bl, V_half, nseg, p, ws, cap, gr, C, W, seg_params_out, counters, w_scalar_total, st,
                        pre, kbeg, kend);
 }
@@ -1247,8 +1317,16 @@ extern "C" int vb_build_keys(const float* u_full, const float* v_full, int n, in
 
 extern "C" size_t vb_stage2_workspace_bytes(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* o) {
   Stage2Plan p{};
-  if (stage2_plan(n_half_total, nseg, npix, o, &p) != VB_OK) return 0;
-  return stage2_workspace(p, nullptr, 0, nullptr);
+  // the pair count is not known here: room for the clusters of any
+  size_t need = 0;
+  if (stage2_plan(n_half_total, nseg, npix, o, &p, 0) != VB_OK) return 0;
+  need = stage2_workspace(p, nullptr, 0, nullptr);
+  for (int64_t nbl = 1; nbl <= n_half_total && nbl <= 4096; ++nbl) {
+    if (n_half_total % nbl != 0) continue;
+    cluster_plan(&p, (int)nbl);
+    need = std::max(need, stage2_workspace(p, nullptr, 0, nullptr));
+  }
+  return need;
 }
 
 extern "C" int vb_recon_batched(const vb_sky* sky, const vb_baselines* bl, const float* V_half, int nseg,
@@ -1259,8 +1337,12 @@ extern "C" int vb_recon_batched(const vb_sky* sky, const vb_baselines* bl, const
   if (bl->nbl <= 0 || bl->n_full % (2 * bl->nbl) != 0) return fail(VB_ERR_INVALID, "vb_recon_batched: n_full/nbl");
   if (!C || !V_half || !seg_t0 || !seg_tlen) return fail(VB_ERR_INVALID, "vb_recon_batched: null buffer");
   Stage2Plan p{};
-  VB_TRY(stage2_plan(bl->n_full / 2, nseg, sky->npix, o, &p));
+  VB_TRY(stage2_plan(bl->n_full / 2, nseg, sky->npix, o, &p, bl->nbl));
   size_t need = stage2_workspace(p, nullptr, 0, nullptr);
+  if (p.trk && ws_bytes < need) {   // without clusters less is needed
+    p.trk = 0;
+    need = stage2_workspace(p, nullptr, 0, nullptr);
+  }
   if (!workspace || ws_bytes < need) return fail(VB_ERR_NOMEM, "vb_recon_batched: workspace %zu < %zu", ws_bytes, need);
   if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
     return fail(VB_ERR_INVALID, "vb_recon_batched: workspace %p is not 256-byte aligned", workspace);

@@ -34,6 +34,7 @@
 #include "vb_geom.cuh"
 #include "vb_internal.h"
 #include "vb_stage1.cuh"
+#include "vb_track.cuh"
 
 namespace vb {
 
@@ -42,8 +43,6 @@ constexpr int TK_SLOTS = 4;
 constexpr int TK_WARPS = 4;              // warps per CTA (independent of one another)
 constexpr int TK_THREADS = 32 * TK_WARPS;
 constexpr int TK_STAGE = 1024;           // chunks hold whole 1024-pixel blocks
-constexpr int TK_LEVELS = 3;             // pixel blocks of 64, 256, 1024
-__host__ __device__ constexpr int tk_block(int level) { return 64 << (2 * level); }
 
 // Polynomial shapes: powers of a in the curve's own factor, in the residuals'
 // first-order terms, and their sum.
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(256) k_track_blocks(const BlockArgs a) {
       ux[k] = uy[k] = uz[k] = 0.0;
       if (base + k < a.npix) {
         x[k] = a.l[base + k]; y[k] = a.m[base + k]; z[k] = a.n[base + k];
-        const float b = a.B[base + k];
+        const float b = a.B ? a.B[base + k] : 0.f;
         const double nn = (double)x[k] * x[k] + (double)y[k] * y[k] + (double)z[k] * z[k];
         bad |= !(fabs(nn - 1.0) <= 4e-6 && fabsf(b) < 1e30f);
         const double inv = rsqrt(nn);
@@ -205,12 +204,6 @@ struct PlanArgs {
   const unsigned* rmax;
   TrackPlan* plan;
 };
-
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 
 // Frame, curve and extents (half-range along the track, curve, residuals from
 // the curve and across) of one sub-group (slots [q0, q0 + ks) of the lanes).
@@ -469,13 +462,6 @@ __global__ void __launch_bounds__(1024) k_track_scan(const TrackPlan* plan, int 
   }
 }
 
-// Sine of the horizon angle of a unit endpoint (NaN where the endpoint is off
-// the unit sphere: no cone test then decides anything).
-__device__ __forceinline__ float horizon_sine(const float4 d) {
-  const double rr = (double)d.x * d.x + (double)d.y * d.y + (double)d.z * d.z;
-  return fabs(rr - 1.0) <= 2e-6 && fabsf(d.w) <= 1.f ? sqrtf(fmaxf(0.f, 1.f - d.w * d.w)) : NAN;
-}
-
 // Lists, and the factored groups' baselines in group order (the steps of one
 // pair are 2 nbl apart in the caller's arrays).
 struct PackArgs {
@@ -557,20 +543,6 @@ __device__ __forceinline__ void phase_cs(double U, double V, double W, float l, 
   const double t = fma(U, (double)l, fma(V, (double)m, fma(W, (double)n, kMagic)));
   const unsigned kb = ((unsigned)__double2loint(t) & 0x7FFFFFu) ^ flip;
   __sincosf(__fmaf_rn(__uint_as_float(kb), kAngScale, -kTwoPiF), &s, &c);
-}
-
-// One step of the transposed reduction: lanes whose bit M is clear keep the
-// first half of the list, the others the second half (an odd list is padded
-// with a zero).
-template <int N, int M>
-__device__ __forceinline__ void fold_half(float* v, bool up) {
-  constexpr int H = (N + 1) / 2;
-#pragma unroll
-  for (int i = 0; i < H; ++i) {
-    const float other = i + H < N ? v[i + H] : 0.f;
-    const float keep = up ? other : v[i], send = up ? v[i] : other;
-    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, M);
-  }
 }
 
 // (l, m, n, B) of pixel p0 + j of a block of np; B = 0 past its end.
@@ -655,61 +627,16 @@ __device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, i
 template <int SET>
 __device__ __forceinline__ float2 track_eval(const float* mom, float a, float b, float c) {
   using S = Shape<SET>;
-  const float2* m = reinterpret_cast<const float2*>(mom);
+  const f2* m = reinterpret_cast<const f2*>(mom);
+  const f2 a2 = f2_make(a, a);
   auto horner = [&](int o, int n) {
-    float2 h = m[o + n - 1];
+    f2 h = m[o + n - 1];
 #pragma unroll
-    for (int i = n - 2; i >= 0; --i) {
-      const float2 t = m[o + i];
-      h.x = fmaf(h.x, a, t.x);
-      h.y = fmaf(h.y, a, t.y);
-    }
+    for (int i = n - 2; i >= 0; --i) h = f2_fma(h, a2, m[o + i]);
     return h;
   };
-  float2 r = horner(0, S::N);
-  const float2 hb = horner(S::N, S::NE), hc = horner(S::N + S::NE, S::NE);
-  r.x = fmaf(b, hb.x, fmaf(c, hc.x, r.x));
-  r.y = fmaf(b, hb.y, fmaf(c, hc.y, r.y));
-  return r;
-}
-
-// cos and sin of t turns in FP64 to about 2e-9 (Taylor series on an eighth of a
-// turn): the factor of a whole block's sum, so it must not carry the SFU's noise.
-__device__ __forceinline__ void turn_cs(double t, double& s, double& c) {
-  const double k = fma(t, 4.0, 6755399441055744.0);   // 1.5 * 2^52: rounds to an integer
-  const int q = __double2loint(k);
-  const double g = fma(k - 6755399441055744.0, -0.25, t);
-  const double x = g * 6.283185307179586476925, x2 = x * x;
-  double sp = fma(x2, 1.0 / 362880.0, -1.0 / 5040.0);
-  sp = fma(sp, x2, 1.0 / 120.0);
-  sp = fma(sp, x2, -1.0 / 6.0);
-  sp = fma(sp * x2, x, x);
-  double cp = fma(x2, -1.0 / 3628800.0, 1.0 / 40320.0);
-  cp = fma(cp, x2, -1.0 / 720.0);
-  cp = fma(cp, x2, 1.0 / 24.0);
-  cp = fma(cp, x2, -0.5);
-  cp = fma(cp, x2, 1.0);
-  const double ss = (q & 1) ? cp : sp, cc = (q & 1) ? sp : cp;
-  s = (q & 2) ? -ss : ss;
-  c = ((q + 1) & 2) ? -cc : cc;
-}
-
-// Class of one unit endpoint (d.w = cos phi, s = sin phi of its horizon) against
-// a node's cone of half-angle alpha, as exact_class in float32: every pixel
-// passes when cos(axis, endpoint) >= cos(phi - alpha), every pixel fails when it
-// is <= cos(phi + alpha).  The margin covers the per-pixel test's evaluation
-// error (2e-6) and this test's own (below 1e-6).
-__device__ __forceinline__ int endpoint_class(const TrackNode& n, const float4 d, float s) {
-  constexpr float kMargin = 1.2e-5f;
-  const float cd = fmaf(n.axis.x, d.x, fmaf(n.axis.y, d.y, n.axis.z * d.z));
-  const float cc = d.w * n.axis.w, ss = s * n.cen.w;
-  const bool vis = n.axis.w >= d.w && cd >= cc + ss + kMargin;
-  const bool hid = n.axis.w >= -d.w && cd <= cc - ss - kMargin;
-  return vis ? kClsVis : (hid ? kClsHid : kClsMix);
-}
-
-__device__ __forceinline__ int both_classes(int e1, int e2) {
-  return (e1 == kClsHid || e2 == kClsHid) ? kClsHid : ((e1 == kClsVis && e2 == kClsVis) ? kClsVis : kClsMix);
+  const f2 h0 = horner(0, S::N), hb = horner(S::N, S::NE), hc = horner(S::N + S::NE, S::NE);
+  return f2_split(f2_fma(f2_make(b, b), hb, f2_fma(f2_make(c, c), hc, h0)));
 }
 
 __device__ __forceinline__ int track_tile_class(const TrackArgs& a, const float4 d1, const float4 d2, int tile) {
@@ -1047,18 +974,23 @@ void track_carve(const Stage1Plan& p, Carve& c, Stage1Buffers& x, bool pixels) {
   }
 }
 
-int track_prepare_pixels(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s) {
-  if (!p.track) return VB_OK;
+int track_nodes(const float* B, const float* l, const float* m, const float* n, int64_t npix, TrackNode* const (&node)[3],
+                unsigned* rmax, cudaStream_t s) {
   BlockArgs k{};
-  k.B = sky->B; k.l = sky->l; k.m = sky->m; k.n = sky->n;
-  k.npix = p.npix;
-  k.nsuper = (int)ceil_div(p.npix, 1024);
-  for (int lev = 0; lev < TK_LEVELS; ++lev) k.node[lev] = b.trk.node[lev];
-  k.rmax = b.trk.rmax;
+  k.B = B; k.l = l; k.m = m; k.n = n;
+  k.npix = npix;
+  k.nsuper = (int)ceil_div(npix, 1024);
+  for (int lev = 0; lev < TK_LEVELS; ++lev) k.node[lev] = node[lev];
+  k.rmax = rmax;
   VB_CUDA(cudaMemsetAsync(k.rmax, 0, TK_LEVELS * sizeof(unsigned), s));
   k_track_blocks<<<std::min(k.nsuper, sm_count() * 16), 256, 0, s>>>(k);
   VB_LAUNCH_CHECK();
   return VB_OK;
+}
+
+int track_prepare_pixels(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s) {
+  if (!p.track) return VB_OK;
+  return track_nodes(sky->B, sky->l, sky->m, sky->n, p.npix, b.trk.node, b.trk.rmax, s);
 }
 
 // Plans the groups and builds both lists; the per-term kernel runs on
