@@ -26,6 +26,7 @@
 #include "vb_geom.cuh"
 #include "vb_internal.h"
 #include "vb_stage2.cuh"
+#include "vb_track.cuh"
 
 namespace vb {
 
@@ -35,9 +36,6 @@ constexpr double kMagic2 = 805306368.0;  // 1.5 * 2^29: 2^-23-turn ulp, see stag
 constexpr float kTwoPiF2 = 6.28318530717958647692f;
 constexpr float kAngScale2 = 6.28318530717958647692f * 1.1920928955078125e-7f;
 
-struct GroupMeta {        // members of a group (member-sampling path)
-  int s0, L, seg, pad;
-};
 
 // --- double-double helpers (Dekker/Knuth two-sum and fma two-product) ------
 struct dd { double hi, lo; };
@@ -231,7 +229,6 @@ struct RecArgs {
   float cosphi;
   int nbl, mirror, blockage, occ_mode;
   GroupRec* rec;
-  GroupMeta* meta;
   unsigned* err;
   const int* dst;       // nullable: place of each group's record (clusters in use)
 };
@@ -292,7 +289,6 @@ __global__ void k_group_records(const RecArgs r, int max_groups) {
       if (!r.mirror && !(isfinite(o.vx) && isfinite(o.vy))) o.flags |= 2;
     }
     r.rec[r.dst ? r.dst[g] : g] = o;
-    if (r.meta) r.meta[g] = GroupMeta{s0, L, seg, 0};
   }
 }
 
@@ -311,7 +307,7 @@ struct ReconArgs {
   int block_pix, nblocks, nchunk_target;
   const int* ngroups;
   const GroupRec* rec;
-  const GroupMeta* meta;
+  const int* start;          // first member of each group
   const vb_seg_params* sp;   // per segment: fa, fb, first group, group count
   const int* svals;
   const float* V;
@@ -771,17 +767,36 @@ __global__ void __launch_bounds__(S2_THREADS, 2) k_recon_rec(const ReconArgs a) 
   }
 }
 
-// occ_mode 0 / 1 / other: per pixel, sample members, average the visible V.
+// occ_mode 0 / 1 / other: per pixel, the visible ones of the group's members (all
+// of them, the first, or four samples) are averaged.
+//
+// Bound: issue.  A step holds up to 64 groups and 256 members in shared memory
+// (gathered once per CTA, where every warp used to fetch each member's endpoints
+// itself), each member classified against the block's cone, so that hidden
+// members are skipped and visible ones take no test; a group without any member
+// left costs no sine.  1.48 -> 0.86 ms (49,152 pixels, four samples, signed set).
+constexpr int M_GROUPS = 64, M_MEMBERS = S2_THREADS, M_PPT = 2;
+struct MemberRec {
+  float4 p1, p2;          // (x, y, z, invn) of the endpoints
+  float c1, c2, vx, vy;
+};
 template <int MODE>
 __global__ void __launch_bounds__(S2_THREADS) k_recon_members(const ReconArgs a) {
-  __shared__ GroupRec s_rec[S2_STAGE];
-  __shared__ GroupMeta s_meta[S2_STAGE];
-  __shared__ int s_item;
+  __shared__ GroupRec s_rec[M_GROUPS];
+  __shared__ MemberRec s_mem[M_MEMBERS];
+  __shared__ int s_cls[M_MEMBERS];
+  __shared__ int s_beg[M_GROUPS + 1];
+  __shared__ float s_red[4][S2_THREADS / 32];
+  __shared__ TrackNode s_node;
+  __shared__ int s_item, s_ngs;
   constexpr bool kDouble = (MODE == VB_PREC_FP64);
+  using Acc = typename std::conditional<kDouble, double, float>::type;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int ng = *a.ngroups;
   const int gchunk = group_chunk(ng, a.nchunk_target);
   const int nchunk = (ng + gchunk - 1) / gchunk;
   const int n_items = nchunk * a.nblocks;
+  const int per = a.occ_mode == 0 ? 0 : (a.occ_mode == 1 ? 1 : 4);   // members a group (0: all)
   unsigned long long c_all = 0;
   for (;;) {
     __syncthreads();
@@ -791,77 +806,169 @@ __global__ void __launch_bounds__(S2_THREADS) k_recon_members(const ReconArgs a)
     if (item >= n_items) break;
     const int gc = item / a.nblocks;
     const int blk = item - gc * a.nblocks;
-    const int64_t pix = (int64_t)blk * a.block_pix + threadIdx.x;
-    const bool active = pix < a.npix;
-    float lf = 0.f, mf = 0.f, nf = 0.f;
-    double ld = 0.0, md = 0.0, nd = 0.0;
-    if (active) {
-      lf = a.l[pix]; mf = a.m[pix]; nf = a.n[pix];
-      ld = lf; md = mf; nd = nf;
+    const int64_t pix0 = (int64_t)blk * a.block_pix;
+    RecPix px[M_PPT];
+    float sx = 0.f, sy = 0.f, sz = 0.f, off = 0.f;
+#pragma unroll
+    for (int q = 0; q < M_PPT; ++q) {
+      const int64_t pix = min(pix0 + q * S2_THREADS + threadIdx.x, a.npix - 1);
+      px[q].lf = a.l[pix]; px[q].mf = a.m[pix]; px[q].nf = a.n[pix];
+      px[q].ld = px[q].lf; px[q].md = px[q].mf; px[q].nd = px[q].nf;
+      sx += px[q].lf; sy += px[q].mf; sz += px[q].nf;
+      const float rr = (float)fabs(px[q].ld * px[q].ld + px[q].md * px[q].md + px[q].nd * px[q].nd - 1.0);
+      off = rr <= off ? off : rr;   // (a NaN stays)
     }
-    const int npx_blk = (int)min((int64_t)a.block_pix, a.npix - (int64_t)blk * a.block_pix);
-    double totC = 0.0;
-    unsigned totW = 0;
+    // the block's cone: axis, then the smallest dot with it
+    auto reduce = [&](float v, int k, bool add) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float t = __shfl_xor_sync(0xffffffffu, v, o);
+        v = add ? v + t : (t < v || t != t ? t : v);
+      }
+      if (lane == 0) s_red[k][warp] = v;
+    };
+    reduce(sx, 0, true);
+    reduce(sy, 1, true);
+    reduce(sz, 2, true);
+    reduce(-off, 3, false);
+    __syncthreads();
+    sx = sy = sz = 0.f;
+    off = 0.f;
+    for (int w = 0; w < S2_THREADS / 32; ++w) {
+      sx += s_red[0][w]; sy += s_red[1][w]; sz += s_red[2][w];
+      off = -s_red[3][w] <= off ? off : -s_red[3][w];
+    }
+    const float inv = rsqrtf(sx * sx + sy * sy + sz * sz);
+    sx *= inv; sy *= inv; sz *= inv;
+    float dmin = 1.f;
+#pragma unroll
+    for (int q = 0; q < M_PPT; ++q) {
+      const float d = px[q].lf * sx + px[q].mf * sy + px[q].nf * sz;
+      dmin = d < dmin || d != d ? d : dmin;
+    }
+    __syncthreads();
+    reduce(dmin, 0, false);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 0; w < S2_THREADS / 32; ++w) dmin = s_red[0][w] < dmin || s_red[0][w] != s_red[0][w] ? s_red[0][w] : dmin;
+      // rounded outwards; pixels off the unit sphere leave every member to the test
+      const float ca = fmaxf(-1.f, dmin - 1e-6f);
+      s_node.axis = make_float4(sx, sy, sz, ca);
+      s_node.cen = make_float4(0.f, 0.f, 0.f, off <= 4e-6f ? sqrtf(fmaxf(0.f, 1.f - ca * ca)) + 1e-6f : NAN);
+    }
+    const int npx_blk = (int)min((int64_t)a.block_pix, a.npix - pix0);
+    double totC[M_PPT];
+    unsigned totW[M_PPT];
+#pragma unroll
+    for (int q = 0; q < M_PPT; ++q) { totC[q] = 0.0; totW[q] = 0u; }
     const int g_begin = gc * gchunk;
     const int g_end = min(ng, g_begin + gchunk);
-    for (int gs = g_begin; gs < g_end; gs += S2_STAGE) {
-      const int nst = min(S2_STAGE, g_end - gs);
-      __syncthreads();
-      for (int j = threadIdx.x; j < nst; j += S2_THREADS) {
-        s_rec[j] = a.rec[gs + j];
-        s_meta[j] = a.meta[gs + j];
+    int gs = g_begin;
+    int done = 0;                          // members of group gs summed by earlier steps (occ_mode 0)
+    float vx[M_PPT], vy[M_PPT];
+    int cnt[M_PPT];
+    while (gs < g_end) {
+      __syncthreads();                     // the previous step is read; the cone is here
+      // this step: groups [gs, gs + ngs), or a part of one group longer than the buffer
+      if (threadIdx.x < M_GROUPS + 1) {
+        const int g = min(gs + (int)threadIdx.x, g_end);
+        s_beg[threadIdx.x] = per ? (g - gs) * per : a.start[g] - a.start[gs] - done;
       }
       __syncthreads();
-      double accd = 0.0;
-      float accf = 0.f;
-      for (int j = 0; j < nst; ++j) {
-        const GroupRec& r = s_rec[j];
-        if (r.flags & 1) continue;
-        const GroupMeta mt = s_meta[j];
-        const int L = mt.L;
-        if (L <= 0) continue;
-        float sx = 0.f, sy = 0.f;
-        int cnt = 0;
-        auto handle = [&](int pos) {
-          const int idx = a.svals[pos];
-          const int f = a.mirror ? half_to_full_pos(idx, a.nbl) : idx;
-          const float o1 = occ_dot(lf, mf, nf, a.x1[f], a.y1[f], a.z1[f], a.in1[f]);
-          const float o2 = occ_dot(lf, mf, nf, a.x2[f], a.y2[f], a.z2[f], a.in2[f]);
-          const float c1 = a.cp1 ? a.cp1[f] : a.cosphi;
-          const float c2 = a.cp2 ? a.cp2[f] : a.cosphi;
-          if (o1 >= c1 && o2 >= c2) {
-            const float vx = a.V[2 * idx], vy = a.V[2 * idx + 1];
-            if (isfinite(vx) && isfinite(vy)) { sx += vx; sy += vy; ++cnt; }
+      if (threadIdx.x == 0) {
+        int n = 0;
+        while (n < M_GROUPS && gs + n < g_end && s_beg[n + 1] <= M_MEMBERS) ++n;
+        s_ngs = n;
+      }
+      __syncthreads();
+      const bool part = s_ngs == 0;
+      const int ngs = part ? 1 : s_ngs;
+      const int nmem = part ? M_MEMBERS : s_beg[ngs];
+      for (int i = threadIdx.x; i < ngs * (int)(sizeof(GroupRec) / 16); i += S2_THREADS)
+        reinterpret_cast<float4*>(s_rec)[i] = reinterpret_cast<const float4*>(a.rec + gs)[i];
+      if ((int)threadIdx.x < nmem) {
+        int pos;
+        if (per == 0) pos = a.start[gs] + done + threadIdx.x;
+        else {
+          const int g = gs + threadIdx.x / per, k = threadIdx.x % per;
+          const int s0 = a.start[g], L = a.start[g + 1] - s0;
+          pos = k == 0 ? s0 : (k == 1 ? s0 + L / 3 : (k == 2 ? s0 + 2 * L / 3 : s0 + L - 1));
+        }
+        const int idx = a.svals[pos];
+        const int f = a.mirror ? half_to_full_pos(idx, a.nbl) : idx;
+        MemberRec m;
+        m.p1 = make_float4(a.x1[f], a.y1[f], a.z1[f], a.in1[f]);
+        m.p2 = make_float4(a.x2[f], a.y2[f], a.z2[f], a.in2[f]);
+        m.c1 = a.cp1 ? a.cp1[f] : a.cosphi;
+        m.c2 = a.cp2 ? a.cp2[f] : a.cosphi;
+        m.vx = a.V[2 * idx];
+        m.vy = a.V[2 * idx + 1];
+        s_mem[threadIdx.x] = m;
+        const float4 d1 = make_float4(m.p1.x * m.p1.w, m.p1.y * m.p1.w, m.p1.z * m.p1.w, m.c1);
+        const float4 d2 = make_float4(m.p2.x * m.p2.w, m.p2.y * m.p2.w, m.p2.z * m.p2.w, m.c2);
+        const int c = both_classes(endpoint_class(s_node, d1, horizon_sine(d1)), endpoint_class(s_node, d2, horizon_sine(d2)));
+        s_cls[threadIdx.x] = isfinite(m.vx) && isfinite(m.vy) ? c : kClsHid;   // a non-finite V is never averaged
+      }
+      __syncthreads();
+      Acc acc[M_PPT];
+#pragma unroll
+      for (int q = 0; q < M_PPT; ++q) acc[q] = Acc(0);
+      for (int j = 0; j < ngs; ++j) {
+        const int m0 = part || j == 0 ? 0 : s_beg[j], m1 = part ? M_MEMBERS : s_beg[j + 1];
+        if (j > 0 || done == 0) {
+#pragma unroll
+          for (int q = 0; q < M_PPT; ++q) { vx[q] = vy[q] = 0.f; cnt[q] = 0; }
+        }
+        for (int i = m0; i < m1; ++i) {
+          const int c = s_cls[i];
+          if (c == kClsHid) continue;
+          const MemberRec m = s_mem[i];
+#pragma unroll
+          for (int q = 0; q < M_PPT; ++q) {
+            bool in = true;
+            if (c == kClsMix)
+              in = occ_dot(px[q].lf, px[q].mf, px[q].nf, m.p1.x, m.p1.y, m.p1.z, m.p1.w) >= m.c1 &&
+                   occ_dot(px[q].lf, px[q].mf, px[q].nf, m.p2.x, m.p2.y, m.p2.z, m.p2.w) >= m.c2;
+            if (in) { vx[q] += m.vx; vy[q] += m.vy; ++cnt[q]; }
           }
-        };
-        const int s0 = mt.s0, s1 = mt.s0 + L;
-        if (a.occ_mode == 0) {
-          for (int pos = s0; pos < s1; ++pos) handle(pos);
-        } else if (a.occ_mode == 1) {
-          handle(s0);
-        } else {
-          handle(s0);
-          handle(s0 + (L / 3));
-          handle(s0 + (2 * L / 3));
-          handle(s1 - 1);
         }
-        if (cnt > 0 && active) {
-          const float invc = 1.0f / (float)cnt;
-          const float vx = sx * invc, vy = sy * invc;
-          float s, c;
+        if (part) continue;                // more members follow
+        const GroupRec& r = s_rec[j];
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < M_PPT; ++q) any |= cnt[q] > 0;
+        if ((r.flags & 1) || !__any_sync(0xffffffffu, any)) continue;
+#pragma unroll
+        for (int q = 0; q < M_PPT; ++q) {
+          const float invc = 1.0f / (float)cnt[q];
+          const float ux = vx[q] * invc, uy = vy[q] * invc;
+          float sn, cs;
           double sd, cd;
-          recon_phase<MODE>(r, ld, md, nd, lf, mf, nf, s, c, sd, cd);
-          if constexpr (kDouble) accd += (double)vx * cd - (double)vy * sd;
-          else accf += fmaf(vx, c, -vy * s);
-          totW += 1;
+          recon_phase<MODE>(r, px[q].ld, px[q].md, px[q].nd, px[q].lf, px[q].mf, px[q].nf, sn, cs, sd, cd);
+          if (cnt[q] > 0) {
+            if constexpr (kDouble) acc[q] += (double)ux * cd - (double)uy * sd;
+            else acc[q] += fmaf(ux, cs, -uy * sn);
+            totW[q] += 1;
+          }
         }
       }
-      totC += kDouble ? accd : (double)accf;
+#pragma unroll
+      for (int q = 0; q < M_PPT; ++q) totC[q] += (double)acc[q];
+      if (part) {
+        done += M_MEMBERS;
+      } else {
+        done = 0;
+        gs += ngs;
+      }
     }
     if (threadIdx.x == 0) c_all += (int64_t)npx_blk * (g_end - g_begin);
-    if (active) {
-      a.Cpart[(int64_t)gc * a.npix + pix] = totC;
-      a.Wpart[(int64_t)gc * a.npix + pix] = totW;
+#pragma unroll
+    for (int q = 0; q < M_PPT; ++q) {
+      const int64_t pix = pix0 + q * S2_THREADS + threadIdx.x;
+      if (pix < a.npix) {
+        a.Cpart[(int64_t)gc * a.npix + pix] = totC[q];
+        a.Wpart[(int64_t)gc * a.npix + pix] = totW[q];
+      }
     }
   }
   if (a.counters && threadIdx.x == 0) {
@@ -948,14 +1055,14 @@ int stage2_plan(int n_half_total, int nseg, int64_t npix, const vb_stage2_opts* 
   q.cull = (o->cull == VB_CULL_EXACT && q.blockage && q.occ_mode == 2) ? VB_CULL_EXACT : VB_CULL_NONE;
   q.grid_res = o->grid_res;
   // pixels per thread of the representative / average path (the member path
-  // keeps one): by default 4 with the FP64 phase in FP32 (its pair records are
+  // has 2): by default 4 with the FP64 phase in FP32 (its pair records are
   // read once per 4 pixels; 0.835 against 0.772 of the SFU peak at nside 1024),
   // 2 in the other modes (whose registers do not hold 4); 1, 2 or 4 on request
   if (o->ppt != 0 && o->ppt != 1 && o->ppt != 2 && o->ppt != 4)
     return fail(VB_ERR_INVALID, "stage 2: ppt=%d (0, 1, 2 or 4)", o->ppt);
   const bool members = q.blockage && q.occ_mode != 2;
   const int ppt_auto = (o->precision == VB_PREC_FP32_FP64PH) ? 4 : 2;
-  q.ppt = members ? 1 : (o->ppt == 0 ? ppt_auto : o->ppt);
+  q.ppt = members ? M_PPT : (o->ppt == 0 ? ppt_auto : o->ppt);
   q.bl_max = o->bl_max;
   q.lambda = o->lambda;
   q.n_half_total = n_half_total;
@@ -998,7 +1105,6 @@ struct S2Slices {
   int *v0, *v1, *flags, *gid, *start, *ngroups, *queue;
   unsigned* err;
   GroupRec* rec;
-  GroupMeta* meta;
   double* Cpart;
   unsigned* Wpart;
   ExactCone* cones;
@@ -1026,7 +1132,6 @@ static size_t carve2(const Stage2Plan& p, void* ws, size_t cap, S2Slices* s) {
   x.queue = c.take<int>(4);
   x.wsum = c.take<double>(2);
   x.rec = c.take<GroupRec>(n);
-  x.meta = c.take<GroupMeta>(n);
   const size_t rows = (size_t)p.nchunk_target + (p.trk ? p.trk_rows : 0);
   x.Cpart = c.take<double>(rows * (size_t)p.npix);
   x.Wpart = c.take<unsigned>(rows * (size_t)p.npix);
@@ -1166,7 +1271,7 @@ int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half
     r.x2 = bl->x2; r.y2 = bl->y2; r.z2 = bl->z2; r.in2 = bl->invn2;
     r.cp1 = bl->cosphi1; r.cp2 = bl->cosphi2; r.cosphi = bl->cosphi;
     r.nbl = nbl; r.mirror = p.mirror; r.blockage = p.blockage; r.occ_mode = p.occ_mode;
-    r.rec = x.rec; r.meta = p.trk ? nullptr : x.meta; r.err = x.err;
+    r.rec = x.rec; r.err = x.err;
     r.dst = p.trk ? x.trk.dst : nullptr;
     k_group_records<<<g, 256, 0, st>>>(r, n);
     VB_LAUNCH_CHECK();
@@ -1179,7 +1284,7 @@ int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half
     ReconArgs ra{};
     ra.l = sky->l; ra.m = sky->m; ra.n = sky->n; ra.npix = p.npix;
     ra.block_pix = p.block_pix; ra.nblocks = p.nblocks; ra.nchunk_target = p.nchunk_target;
-    ra.ngroups = x.ngroups; ra.rec = x.rec; ra.meta = x.meta; ra.sp = x.sp; ra.svals = sv; ra.V = Vk;
+    ra.ngroups = x.ngroups; ra.rec = x.rec; ra.start = x.start; ra.sp = x.sp; ra.svals = sv; ra.V = Vk;
     ra.x1 = bl->x1; ra.y1 = bl->y1; ra.z1 = bl->z1; ra.in1 = bl->invn1;
     ra.x2 = bl->x2; ra.y2 = bl->y2; ra.z2 = bl->z2; ra.in2 = bl->invn2;
     ra.cp1 = bl->cosphi1; ra.cp2 = bl->cosphi2; ra.cosphi = bl->cosphi;
