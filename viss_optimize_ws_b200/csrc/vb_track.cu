@@ -569,9 +569,9 @@ __device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, i
 #pragma unroll
   for (int c = 0; c < 3; ++c) e[c] = fmaf(sub.gamma, e[3 + c], e[c]);
   const float kq = sub.kappa * inv_r * 0.31830988618379067f;   // 2 kappa / (2 pi r)
-  float v[2 * S::J];
+  f2 v2[S::J];   // (re, im)
 #pragma unroll
-  for (int i = 0; i < 2 * S::J; ++i) v[i] = 0.f;
+  for (int i = 0; i < S::J; ++i) v2[i] = 0ull;
   // odd pixels half a turn on with a negated brightness, as in the per-term kernel
   const unsigned flip = (lane & 1) ? 0x4B400000u : 0x4B000000u;
   float4 f = pixel_at(ta, p0, np, lane);
@@ -586,16 +586,15 @@ __device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, i
     const float eta = fmaf(dx, e[3], fmaf(dy, e[4], dz * e[5]));
     const float zet = fmaf(dx, e[6], fmaf(dy, e[7], dz * e[8]));
     const float q = kq * eta;
+    const f2 eta2 = f2_make(eta, eta), zet2 = f2_make(zet, zet);
     float r0 = 0.f, i0 = 0.f, r1 = zr * Bp, i1 = zi * Bp;   // g_{n-1}, g_n
 #pragma unroll
     for (int n = 0; n < S::N; ++n) {
-      v[2 * n] += r1;
-      v[2 * n + 1] += i1;
+      const f2 g = f2_make(r1, i1);
+      v2[n] = f2_add(v2[n], g);
       if (n < S::NE) {
-        v[2 * (S::N + n)] = fmaf(eta, r1, v[2 * (S::N + n)]);
-        v[2 * (S::N + n) + 1] = fmaf(eta, i1, v[2 * (S::N + n) + 1]);
-        v[2 * (S::N + S::NE + n)] = fmaf(zet, r1, v[2 * (S::N + S::NE + n)]);
-        v[2 * (S::N + S::NE + n) + 1] = fmaf(zet, i1, v[2 * (S::N + S::NE + n) + 1]);
+        v2[S::N + n] = f2_fma(eta2, g, v2[S::N + n]);
+        v2[S::N + S::NE + n] = f2_fma(zet2, g, v2[S::N + S::NE + n]);
       }
       if (n + 1 < S::N) {
         const float nq = (float)n * q;
@@ -606,6 +605,13 @@ __device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, i
       }
     }
     f = next;
+  }
+  float v[2 * S::J];
+#pragma unroll
+  for (int i = 0; i < S::J; ++i) {
+    const float2 t = f2_split(v2[i]);
+    v[2 * i] = t.x;
+    v[2 * i + 1] = t.y;
   }
   constexpr int N = 2 * S::J, N1 = N / 2, N2 = N / 4, N3 = N / 8, N4 = N / 16, N5 = (N4 + 1) / 2;
   fold_half<N, 16>(v, lane & 16);
