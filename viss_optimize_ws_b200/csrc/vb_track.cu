@@ -42,7 +42,8 @@ constexpr int TK_GROUP = kTrackGroup;    // slots of a group: 4 per lane
 constexpr int TK_SLOTS = 4;
 constexpr int TK_WARPS = 4;              // warps per CTA (independent of one another)
 constexpr int TK_THREADS = 32 * TK_WARPS;
-constexpr int TK_STAGE = 1024;           // chunks hold whole 1024-pixel blocks
+constexpr int TK_QUAD = 4;               // blocks whose moments a warp forms at a time, 8 lanes each
+constexpr int TK_CHUNK = TK_QUAD * 1024; // chunks hold whole quads of the largest blocks
 
 // Polynomial shapes: powers of a in the curve's own factor, in the residuals'
 // first-order terms, and their sum.
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(256) k_track_blocks(const BlockArgs a) {
 // Plan: the shape of each group (slots per sub-group, pixel block, polynomial),
 // or none.  One warp per group; O(n_half).
 struct PlanArgs {
-  const float *u, *v, *w;
+  const float *u, *v, *w, *x1, *y1, *z1, *in1;
   int nbl, steps, gpp, ngroups, max_level, blockage;
   const unsigned* rmax;
   TrackPlan* plan;
@@ -366,11 +367,25 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
   float e[9], R[4], gamma, kappa;
   if (__all_sync(0xffffffffu, fine)) {
     // Issue cycles of a warp for each 32 terms, from the instruction counts of
-    // k_track_sum: pixel step, reduction, evaluation; undecided (baseline,
-    // block) pairs grow with the block's radius.  The per-term kernel takes
-    // about 20 for each 32 terms.
-    const float c_pix[TK_SETS] = {90.f, 130.f, 260.f}, c_red[TK_SETS] = {170.f, 240.f, 480.f}, c_eval[TK_SETS] = {125.f, 145.f, 240.f};
-    float best = 12.f;
+    // k_track_sum: pixel steps, reduction, evaluation; and what the blocks on the
+    // horizon cost more: a quad of each lower level, and 64-pixel parts term by
+    // term for the steps that the horizon crosses there.  It sweeps `turn` radians
+    // over the group (the first endpoint's motion), so that a share of the visible
+    // blocks in proportion to turn + 2 r lies on it; the factor 0.28 and the line at
+    // 10 were measured over nside 256 to 1024, lunar and Earth orbits, days 1 to 8
+    // (0.14 to 1.1 and 7 to 15 tried: within 15 % of the best shape in each).  The
+    // per-term kernel takes about 18 cycles for each 32 terms, and this one issues
+    // 0.6 to 0.7 instructions a cycle.
+    const float c_pix[TK_SETS] = {90.f, 130.f, 170.f}, c_red[TK_SETS] = {50.f, 70.f, 95.f}, c_eval[TK_SETS] = {125.f, 145.f, 165.f};
+    float turn = 0.f;
+    if (a.blockage) {
+      const int64_t i0 = (int64_t)s0 * 2 * a.nbl + pair, i1 = (int64_t)(s0 + nv - 1) * 2 * a.nbl + pair;
+      const float k0 = a.in1[i0], k1 = a.in1[i1];
+      const float dx = a.x1[i1] * k1 - a.x1[i0] * k0, dy = a.y1[i1] * k1 - a.y1[i0] * k0, dz = a.z1[i1] * k1 - a.z1[i0] * k0;
+      turn = sqrtf(dx * dx + dy * dy + dz * dz) / (float)max(nv - 1, 1);   // a step
+    }
+    const float r64 = __uint_as_float(a.rmax[0]);
+    float best = 10.f;
     for (int ls = 0; ls <= 2; ++ls) {
       const int ks = 1 << ls;
       float M[4] = {0.f, 0.f, 0.f, 0.f};
@@ -380,6 +395,7 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
       }
       bool fits = false;
       const float fill = (float)nv / (float)(ks * 32 * ((nv + ks * 32 - 1) / (ks * 32)));
+      const float crossed = fminf(32.f * ks, 1.f + 2.f * r64 / fmaxf(turn, 1e-6f));   // steps on the horizon in a 64-pixel part
       for (int lev = 0; lev <= a.max_level; ++lev) {
         const float r = __uint_as_float(a.rmax[lev]);
         const float k = 6.2831855f * r, E = k * (M[2] + M[3]);
@@ -389,8 +405,11 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
           if (!(h[set][0] + E * h[set][1] <= kTailMax && E <= kResidualMax)) continue;
           fits = true;
           const float P = (float)tk_block(lev);
-          const float cost = (P * (1.f / 32.f) * c_pix[set] + c_red[set] + ks * c_eval[set]) / (ks * P * fill) +
-                             (a.blockage ? 10.f * r : 0.f);
+          float node = P * (1.f / 32.f) * c_pix[set] + c_red[set] + ks * c_eval[set];
+          if (a.blockage)
+            node += fminf(1.f, 0.28f * (turn * 32.f * ks + 2.f * r)) *
+                    (lev * (P * (1.f / 32.f) * c_pix[set] + 4.f * (c_red[set] + c_eval[set])) + P * (1.f / 64.f) * (150.f + 70.f * crossed));
+          const float cost = node / (ks * P * fill);
           if (cost < best) { best = cost; mode = set | (ls << 4) | (lev << 8); }
         }
       }
@@ -518,9 +537,9 @@ __global__ void __launch_bounds__(128) k_track_pack(const PackArgs a) {
 __device__ __forceinline__ int cls_get(int c, int q) { return (c >> (2 * q)) & 3; }
 __device__ __forceinline__ int cls_put(int c, int q, int v) { return (c & ~(3 << (2 * q))) | (v << (2 * q)); }
 
-// Included baselines of a sub-group up to which a 64-pixel part of a block is
-// summed term by term rather than through its moments.
-constexpr int kFewVisible = 20;
+// Included (baseline, block) pairs of a sub-group up to which four 64-pixel parts
+// of a block are summed term by term rather than through their moments.
+constexpr int kFewVisible = 24;
 
 struct TrackWarp {               // one warp's group
   double2 acc[TK_SLOTS][32];
@@ -528,7 +547,7 @@ struct TrackWarp {               // one warp's group
   float a[TK_SLOTS][32], b[TK_SLOTS][32], c[TK_SLOTS][32];
   float4 d1[TK_SLOTS][32], d2[TK_SLOTS][32];
   float s1[TK_SLOTS][32], s2[TK_SLOTS][32];
-  float mom[2 * TK_JMAX];
+  float mom[TK_QUAD][2 * TK_JMAX];
   TrackPlan plan;
 };
 struct TrackSmem {
@@ -545,22 +564,26 @@ __device__ __forceinline__ void phase_cs(double U, double V, double W, float l, 
   __sincosf(__fmaf_rn(__uint_as_float(kb), kAngScale, -kTwoPiF), &s, &c);
 }
 
-// (l, m, n, B) of pixel p0 + j of a block of np; B = 0 past its end.
+// (l, m, n, B) of pixel p0 + j of a block of np; B = 0 past its end (and the
+// position of some pixel of the sky).
 __device__ __forceinline__ float4 pixel_at(const TrackArgs& a, int64_t p0, int np, int j) {
-  const int64_t p = p0 + (j < np ? j : np - 1);
+  const int64_t p = min(p0 + (j < np ? j : 0), a.npix - 1);
   return make_float4(__ldg(a.l + p), __ldg(a.m + p), __ldg(a.n + p), j < np ? __ldg(a.B + p) : 0.f);
 }
 
-// Moments of one (sub-group, block) into the warp's shared-memory slots, scaled
-// by their coefficients.  With q = 2 kappa eta / (2 pi r) the generating function
+// Moments of one sub-group over four neighbouring blocks (lane >> 3 is the
+// lane's block, p0, np, cen its pixels and centre) into the warp's shared-memory
+// slots, scaled by their coefficients.  Eight lanes a block: the transposed
+// reduction of 2 J values then costs 7/8 N shuffles for four blocks instead of
+// 31/32 N for each (a quarter of a 64-pixel block's time, 8 % of a 256-pixel one).  With q = 2 kappa eta / (2 pi r) the generating function
 // e^{i (a tau + a^2 q / 2)} = sum_n (i a)^n g_n / n! has
 //   g_n = tau g_{n-1} - i (n - 1) q g_{n-2},
 // so that the curve costs five operations a power and the moments of z g_n
 // (and, for the first half of them, of z g_n eta and z g_n zeta: the residuals
 // from the curve to first order) are all that the block contributes.
 template <int SET>
-__device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, int np, const TrackSub& sub, const float4 cen, float inv_r,
-                                              const float* scale, const unsigned char* dest, float* mom, int lane) {
+__device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, int np, int P, const TrackSub& sub, const float4 cen,
+                                              float inv_r, const float* scale, const unsigned char* dest, float* mom, int lane) {
   using S = Shape<SET>;
   const double U = sub.uc[0], V = sub.uc[1], W = sub.uc[2];
   float e[9];
@@ -574,10 +597,11 @@ __device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, i
   for (int i = 0; i < S::J; ++i) v2[i] = 0ull;
   // odd pixels half a turn on with a negated brightness, as in the per-term kernel
   const unsigned flip = (lane & 1) ? 0x4B400000u : 0x4B000000u;
-  float4 f = pixel_at(ta, p0, np, lane);
+  const int l8 = lane & 7;
+  float4 f = pixel_at(ta, p0, np, l8);
 #pragma unroll 1
-  for (int j0 = 0; j0 < np; j0 += 32) {
-    const float4 next = pixel_at(ta, p0, np, j0 + 32 + lane);   // loaded while this step computes
+  for (int j0 = 0; j0 < P; j0 += 8) {
+    const float4 next = pixel_at(ta, p0, np, j0 + 8 + l8);   // loaded while this step computes
     float zi, zr;
     phase_cs(U, V, W, f.x, f.y, f.z, flip, zi, zr);
     const float Bp = (lane & 1) ? -f.w : f.w;
@@ -613,18 +637,14 @@ __device__ __forceinline__ void track_moments(const TrackArgs& ta, int64_t p0, i
     v[2 * i] = t.x;
     v[2 * i + 1] = t.y;
   }
-  constexpr int N = 2 * S::J, N1 = N / 2, N2 = N / 4, N3 = N / 8, N4 = N / 16, N5 = (N4 + 1) / 2;
-  fold_half<N, 16>(v, lane & 16);
-  fold_half<N1, 8>(v, lane & 8);
-  fold_half<N2, 4>(v, lane & 4);
-  fold_half<N3, 2>(v, lane & 2);
-  fold_half<N4, 1>(v, lane & 1);
-  const int base = ((lane & 16) ? N1 : 0) + ((lane & 8) ? N2 : 0) + ((lane & 4) ? N3 : 0) + ((lane & 2) ? N4 : 0) +
-                   ((lane & 1) ? N5 : 0);
-  __syncwarp();   // the previous block's moments are read
+  constexpr int N = 2 * S::J;
+  fold_half<N, 4>(v, lane & 4);
+  fold_half<N / 2, 2>(v, lane & 2);
+  fold_half<N / 4, 1>(v, lane & 1);
+  const int base = ((lane & 4) ? N / 2 : 0) + ((lane & 2) ? N / 4 : 0) + ((lane & 1) ? N / 8 : 0);
+  __syncwarp();   // the previous moments are read
 #pragma unroll
-  for (int k = 0; k < N5; ++k)
-    if (k < N4 / 2 || (k < N5 && !(lane & 1))) mom[dest[base + k]] = v[k] * scale[base + k];
+  for (int k = 0; k < N / 8; ++k) mom[(lane >> 3) * 2 * TK_JMAX + dest[base + k]] = v[k] * scale[base + k];
   __syncwarp();
 }
 
@@ -672,8 +692,11 @@ __device__ __forceinline__ void track_add(const TrackArgs& a, TrackWarp& w, int 
 // terms are z_p e^{i (a tau + b eta + c zeta)} with an exact small angle.  Out of
 // line: a few per cent of the terms, whose registers the moment loop does not
 // have.
-__device__ __noinline__ void track_terms(const TrackArgs& a, TrackWarp& w, int64_t p0, int np, int cls, const float4 cen, float inv_r,
+__device__ __forceinline__ void track_terms(const TrackArgs& a, int64_t p0, int np, int cls, const float4 cen, float inv_r,
                                          int ks, int64_t o0, int lane) {
+  // (from its own declaration: through a reference the accesses would be generic)
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TrackWarp& w = reinterpret_cast<TrackSmem*>(smem_raw)->w[threadIdx.x >> 5];
   const float kr = 6.28318530717958647692f / inv_r;
   const unsigned flip = (lane & 1) ? 0x4B400000u : 0x4B000000u;
   float4 f[2];
@@ -747,6 +770,83 @@ __device__ __noinline__ void track_terms(const TrackArgs& a, TrackWarp& w, int64
   }
 }
 
+// One step of the walk down the pixel blocks: four neighbouring blocks of level
+// lev from pixel `base` (up to `end`), cls4 the slots' classes in each (a byte a
+// block; slots that other blocks decide are hidden).  Baselines still undecided
+// are classified against each block's cone; the included ones take the blocks'
+// moments; the undecided ones are returned for the blocks' own four parts, or at
+// 64 pixels take the per-pixel test.  A few included baselines in parts of 64
+// pixels are summed term by term with those (not at the group's own level, where
+// a tile that the upstream's cone test calls visible takes no test).
+__device__ __forceinline__ unsigned track_quad(const TrackArgs& a, TrackSmem& sm, TrackWarp& w, int lev, bool top, int set, int ks,
+                                            unsigned cls4, int64_t base, int64_t end, float inv_r, int64_t o0, int lane) {
+  const int P = tk_block(lev);
+  unsigned open4 = 0, rest4 = 0;
+  if (a.blockage) {
+#pragma unroll 1
+    for (int n = 0; n < TK_QUAD; ++n) {
+      const int64_t p0 = base + n * P;
+      int c = (cls4 >> (8 * n)) & 255;
+      if (p0 >= end) c = 0;
+      if (__any_sync(0xffffffffu, c != 0)) {
+        const TrackNode nd = a.node[lev][p0 / P];
+#pragma unroll
+        for (int q = 0; q < TK_SLOTS; ++q)
+          if (cls_get(c, q) == kClsMix)
+            c = cls_put(c, q, both_classes(endpoint_class(nd, w.d1[q][lane], w.s1[q][lane]),
+                                           endpoint_class(nd, w.d2[q][lane], w.s2[q][lane])));
+      }
+      cls4 = (cls4 & ~(255u << (8 * n))) | ((unsigned)c << (8 * n));
+    }
+    // undecided slots (class 2: the high bit of each pair)
+    static_assert(kClsMix == 2 && kClsVis == 1, "class bits");
+    open4 = cls4 & 0xAAAAAAAAu;
+  }
+  unsigned vis4 = cls4 & 0x55555555u;
+  if (end < base + TK_QUAD * P && !a.blockage)
+    for (int n = 0; n < TK_QUAD; ++n)
+      if (base + n * P >= end) vis4 &= ~(255u << (8 * n));
+  const int64_t mine = base + (lane >> 3) * P;
+  const int np = (int)max((int64_t)0, min((int64_t)P, end - mine));
+  const float4 cen = a.node[lev][min(mine, end - 1) / P].cen;
+  for (int q0 = 0; q0 < TK_SLOTS; q0 += ks) {
+    const unsigned slots = ((1u << (2 * ks)) - 1u) << (2 * q0);
+    const unsigned take = vis4 & (slots * 0x01010101u);
+    if (!__any_sync(0xffffffffu, take != 0)) continue;
+    if (lev == 0 && !top && __reduce_add_sync(0xffffffffu, (unsigned)__popc(take)) <= kFewVisible) {
+      rest4 |= take;
+      continue;
+    }
+    const TrackSub& sub = w.plan.sub[q0 / ks];
+    if (set == 0) track_moments<0>(a, mine, np, P, sub, cen, inv_r, sm.scale[0], sm.dest[0], w.mom[0], lane);
+    else if (set == 1) track_moments<1>(a, mine, np, P, sub, cen, inv_r, sm.scale[1], sm.dest[1], w.mom[0], lane);
+    else track_moments<2>(a, mine, np, P, sub, cen, inv_r, sm.scale[2], sm.dest[2], w.mom[0], lane);
+#pragma unroll 1
+    for (int q = q0; q < q0 + ks; ++q) {
+      const float ka = w.a[q][lane], kb = w.b[q][lane], kc = w.c[q][lane];
+#pragma unroll 1
+      for (int n = 0; n < TK_QUAD; ++n) {
+        const bool in = (take >> (8 * n + 2 * q)) & 1u;
+        if (!in) continue;
+        const float2 h = set == 0   ? track_eval<0>(w.mom[n], ka, kb, kc)
+                         : set == 1 ? track_eval<1>(w.mom[n], ka, kb, kc)
+                                    : track_eval<2>(w.mom[n], ka, kb, kc);
+        track_add(a, w, q, lane, a.node[lev][(base + n * P) / P].cen, o0 + q * 32, h.x, h.y);
+      }
+    }
+  }
+  if (lev > 0) return open4;
+  rest4 |= open4;
+#pragma unroll 1
+  for (int n = 0; n < TK_QUAD; ++n) {
+    const int c = (rest4 >> (8 * n)) & 255;
+    if (!__any_sync(0xffffffffu, c != 0)) continue;
+    const int64_t p0 = base + n * P;
+    track_terms(a, p0, (int)min((int64_t)P, end - p0), c, a.node[0][p0 / P].cen, inv_r, ks, o0, lane);
+  }
+  return 0;
+}
+
 __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_constant__ TrackArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TrackSmem& sm = *reinterpret_cast<TrackSmem*>(smem_raw);
@@ -810,87 +910,60 @@ __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_consta
       __syncwarp();
     }
     const int P = tk_block(level);
-    auto refine = [&](int c, const TrackNode* np_) {
-      const TrackNode nd = *np_;
-#pragma unroll
-      for (int q = 0; q < TK_SLOTS; ++q)
-        if (cls_get(c, q) == kClsMix)
-          c = cls_put(c, q, both_classes(endpoint_class(nd, w.d1[q][lane], w.s1[q][lane]),
-                                         endpoint_class(nd, w.d2[q][lane], w.s2[q][lane])));
-      return c;
-    };
     const bool tc = a.tilecone && a.blockage;
     int tcls = act, tile = -1;
 
     const int64_t p_begin = (int64_t)chunk * a.chunk_pix;
     const int64_t p_end = min(a.npix, p_begin + a.chunk_pix);
-    for (int64_t p0 = p_begin; p0 < p_end; p0 += P) {
-      const int np = (int)min((int64_t)P, p_end - p0);
+    for (int64_t p0 = p_begin; p0 < p_end; p0 += TK_QUAD * P) {
+      unsigned cls4 = (unsigned)act * 0x01010101u;
       if (tc) {   // class of the cull tile, as the upstream decides it
-        const int t = (int)(p0 / a.cull_tile);
-        if (t != tile) {
-          tile = t;
-          tcls = act;
+        cls4 = 0;
+        for (int n = 0; n < TK_QUAD; ++n) {
+          const int64_t pn = p0 + n * P;
+          if (pn >= p_end) break;
+          const int t = (int)(pn / a.cull_tile);
+          if (t != tile) {
+            tile = t;
+            tcls = act;
 #pragma unroll
-          for (int q = 0; q < TK_SLOTS; ++q)
-            if (cls_get(tcls, q) != kClsHid)
-              tcls = cls_put(tcls, q, track_tile_class(a, w.d1[q][lane], w.d2[q][lane], t));
+            for (int q = 0; q < TK_SLOTS; ++q)
+              if (cls_get(tcls, q) != kClsHid)
+                tcls = cls_put(tcls, q, track_tile_class(a, w.d1[q][lane], w.d2[q][lane], t));
+          }
+          cls4 |= (unsigned)tcls << (8 * n);
         }
       }
-      // The block, and below it the parts of it that some baselines leave
-      // undecided, down to 64 pixels: (lev, off) walks the block's tree.  At
-      // each node the baselines still open there are classified against the
-      // node's cone; the included ones take the node's moments, the undecided
-      // ones go down, and at 64 pixels to the per-pixel test.
-      int lev = level, off = 0, open1 = 0, open0 = 0;
-      while (off < np) {
-        const int PL = tk_block(lev);
-        const int nb = min(PL, np - off);
-        const int64_t blk = (p0 + off) / PL;
-        int cls = lev == level ? tcls : (lev == 1 ? open1 : open0);
-        if (a.blockage) cls = refine(cls, a.node[lev] + blk);
-        const float4 cen = a.node[lev][blk].cen;
-
-        int rest = 0, kids = 0;   // term by term here; undecided in the children
-        for (int q0 = 0; q0 < TK_SLOTS; q0 += ks) {
-          int nvis = 0;
-          for (int q = q0; q < q0 + ks; ++q) {
-            const int c = cls_get(cls, q);
-            nvis += __popc(__ballot_sync(0xffffffffu, c == kClsVis));
-            if (c == kClsMix) {
-              if (lev) kids = cls_put(kids, q, kClsMix);
-              else rest = cls_put(rest, q, kClsMix);
-            }
-          }
-          if (nvis == 0) continue;
-          if (lev == 0 && level > 0 && nvis <= kFewVisible) {
-            for (int q = q0; q < q0 + ks; ++q)
-              if (cls_get(cls, q) == kClsVis) rest = cls_put(rest, q, kClsVis);
-            continue;
-          }
-          const TrackSub& sub = w.plan.sub[q0 / ks];
-          if (set == 0) track_moments<0>(a, p0 + off, nb, sub, cen, inv_r, sm.scale[0], sm.dest[0], w.mom, lane);
-          else if (set == 1) track_moments<1>(a, p0 + off, nb, sub, cen, inv_r, sm.scale[1], sm.dest[1], w.mom, lane);
-          else track_moments<2>(a, p0 + off, nb, sub, cen, inv_r, sm.scale[2], sm.dest[2], w.mom, lane);
-#pragma unroll 1
-          for (int q = q0; q < q0 + ks; ++q) {
-            if (cls_get(cls, q) != kClsVis) continue;
-            const float ka = w.a[q][lane], kb = w.b[q][lane], kc = w.c[q][lane];
-            const float2 h = set == 0   ? track_eval<0>(w.mom, ka, kb, kc)
-                             : set == 1 ? track_eval<1>(w.mom, ka, kb, kc)
-                                        : track_eval<2>(w.mom, ka, kb, kc);
-            track_add(a, w, q, lane, cen, o0 + q * 32, h.x, h.y);
-          }
+      // walk down: the quad at the group's level, then the four parts of each
+      // block that some baselines leave undecided (one call site: the code of a
+      // quad is most of the kernel's, and shared memory must stay visible as such)
+      int lev = level;
+      int64_t base = p0, end = p_end;
+      unsigned open2 = 0, open1 = 0;   // undecided slots of the blocks of level 2 and 1 still to walk
+      int64_t base1 = p0;
+      for (;;) {
+        const unsigned open = track_quad(a, sm, w, lev, lev == level, set, ks, cls4, base, end, inv_r, o0, lane);
+        if (lev == 2) open2 = open;
+        if (lev == 1) { open1 = open; base1 = base; }
+        const unsigned any1 = __reduce_or_sync(0xffffffffu, open1);
+        const unsigned any2 = __reduce_or_sync(0xffffffffu, open2);
+        if (any1) {
+          const int n = (__ffs(any1) - 1) >> 3;
+          base = base1 + n * tk_block(1);
+          end = min(p_end, base + tk_block(1));
+          cls4 = ((open1 >> (8 * n)) & 255u) * 0x01010101u;
+          open1 &= ~(255u << (8 * n));
+          lev = 0;
+        } else if (any2) {
+          const int n = (__ffs(any2) - 1) >> 3;
+          base = p0 + n * tk_block(2);
+          end = min(p_end, base + tk_block(2));
+          cls4 = ((open2 >> (8 * n)) & 255u) * 0x01010101u;
+          open2 &= ~(255u << (8 * n));
+          lev = 1;
+        } else {
+          break;
         }
-        if (__any_sync(0xffffffffu, rest != 0)) track_terms(a, w, p0 + off, nb, rest, cen, inv_r, ks, o0, lane);
-        if (__any_sync(0xffffffffu, kids != 0)) {
-          if (lev == 2) open1 = kids;
-          else open0 = kids;
-          --lev;
-          continue;
-        }
-        off += PL;
-        while (lev < level && (off & (tk_block(lev + 1) - 1)) == 0) ++lev;
       }
     }
     for (int q = 0; q < TK_SLOTS; ++q) {
@@ -946,8 +1019,8 @@ void track_plan(Stage1Plan* p, int items_per_cta) {
   // the queue's tail stays short, chunks of 4096 pixels at least
   const int64_t warps = (int64_t)sm_count() * 12;
   int64_t nchunk = ceil_div(warps * (items_per_cta > 0 ? std::min(items_per_cta, 48) : 40), ng);
-  nchunk = std::max<int64_t>(1, std::min<int64_t>(nchunk, ceil_div(p->npix, 4 * TK_STAGE)));
-  const int64_t chunk = ceil_div(ceil_div(p->npix, nchunk), TK_STAGE) * TK_STAGE;
+  nchunk = std::max<int64_t>(1, std::min<int64_t>(nchunk, ceil_div(p->npix, TK_CHUNK)));
+  const int64_t chunk = ceil_div(ceil_div(p->npix, nchunk), TK_CHUNK) * TK_CHUNK;
   if (chunk > INT32_MAX / 2 || ng * ceil_div(p->npix, chunk) > INT32_MAX) return;
   p->trk_chunk_pix = (int)chunk;
   p->trk_nchunk = (int)ceil_div(p->npix, chunk);
@@ -1005,6 +1078,7 @@ int track_prepare_pixels(const vb_sky* sky, const Stage1Plan& p, const Stage1Buf
 int track_group(const vb_baselines* bl, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s) {
   PlanArgs k{};
   k.u = bl->u; k.v = bl->v; k.w = bl->w;
+  k.x1 = bl->x1; k.y1 = bl->y1; k.z1 = bl->z1; k.in1 = bl->invn1;
   k.nbl = p.nbl; k.steps = p.trk_steps; k.gpp = p.trk_gpp; k.ngroups = p.trk_groups; k.max_level = p.trk_level;
   k.blockage = p.blockage;
   k.rmax = b.trk.rmax;
@@ -1032,7 +1106,7 @@ int track_sum(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cu
   TrackArgs a{};
   a.B = sky->B; a.l = sky->l; a.m = sky->m; a.n = sky->n; a.npix = p.npix;
   a.chunk_pix = p.trk_chunk_pix; a.nchunk = p.trk_nchunk;
-  a.tilecone = p.cull == VB_CULL_TILECONE; a.cull_tile = a.tilecone ? p.cull_tile : TK_STAGE;
+  a.tilecone = p.cull == VB_CULL_TILECONE; a.cull_tile = p.cull_tile;
   a.mask_visible = p.mask_visible; a.blockage = p.blockage; a.raw = p.phase_corrected ? 0 : 1;
   a.tcx = sky->cx; a.tcy = sky->cy; a.tcz = sky->cz; a.tcosA = sky->cosA; a.tsinA = sky->sinA;
   for (int lev = 0; lev < TK_LEVELS; ++lev) a.node[lev] = b.trk.node[lev];
