@@ -173,11 +173,16 @@ k_exact_cone_meta(int tile_pix, const float* __restrict__ l, const float* __rest
     int64_t rem = npix - p0;
     int tileN = (int)(rem < tile_pix ? rem : tile_pix);
     double sx = 0, sy = 0, sz = 0;
+    bool off_unit = false;
     for (int k = t; k < tileN; k += kMetaThreads) {
       double a = l[p0 + k], b = m[p0 + k], c = n[p0 + k];
-      double inv = 1.0 / sqrt(a * a + b * b + c * c);
+      const double nn = a * a + b * b + c * c;
+      off_unit |= !(fabs(nn - 1.0) <= 1e-5);
+      double inv = 1.0 / sqrt(nn);
       sx += a * inv; sy += b * inv; sz += c * inv;
     }
+    // a pixel vector off the unit sphere: no class can be proven from the cone
+    const bool open = __syncthreads_or(off_unit ? 1 : 0);
     rx[t] = sx; ry[t] = sy; rz[t] = sz;
     __syncthreads();
     for (int off = kMetaThreads >> 1; off > 0; off >>= 1) {
@@ -200,7 +205,7 @@ k_exact_cone_meta(int tile_pix, const float* __restrict__ l, const float* __rest
       __syncthreads();
     }
     if (t == 0) {
-      const double alpha = acos(fmax(-1.0, fmin(1.0, rx[0]))) + 1e-9;
+      const double alpha = open ? 3.14159265358979323846 : acos(fmax(-1.0, fmin(1.0, rx[0]))) + 1e-9;
       ExactCone e;
       e.cx = ccx; e.cy = ccy; e.cz = ccz;
       e.cos_a = cos(alpha);
@@ -209,6 +214,93 @@ k_exact_cone_meta(int tile_pix, const float* __restrict__ l, const float* __rest
       out[tile] = e;
     }
     __syncthreads();
+  }
+}
+
+// Stage-1 pixel records ((l, m) as FP64, (n as FP64 bits, B, n - 1), (l, m, n, B)),
+// and the cones of the sub-tiles (128 or 256 pixels) and of the
+// 1024-pixel tiles where asked for, in one pass and one launch: 4 pixels per
+// thread, so that a warp holds a 128-pixel sub-tile.  A stage-1 call on a small
+// sky spends a third of its time in the launches before the sum (12,288 pixels
+// with 128-pixel cones: 4.3 + 8.4 us as two kernels).
+__global__ void __launch_bounds__(256)
+k_pack_cones(const float* __restrict__ B, const float* __restrict__ l, const float* __restrict__ m,
+             const float* __restrict__ n, int64_t npix, int nsuper, PixRec* __restrict__ px, ExactCone* __restrict__ sub,
+             int sub_warps, ExactCone* __restrict__ tile, int* __restrict__ queue) {
+  __shared__ double s_sum[8][3], s_min[2][8];
+  __shared__ int s_bad[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (queue && blockIdx.x == 0 && threadIdx.x < 4) queue[threadIdx.x] = 0;
+  for (int sb = blockIdx.x; sb < nsuper; sb += gridDim.x) {
+    const int64_t base = (int64_t)sb * 1024 + warp * 128 + lane;
+    double ux[4], uy[4], uz[4], sum[3] = {0.0, 0.0, 0.0};
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      ux[k] = uy[k] = uz[k] = 0.0;
+      const int64_t p = base + 32 * k;
+      if (p >= npix) continue;
+      const float lf = l[p], mf = m[p], nf = n[p], bf = B[p];
+      const double ld = lf, md = mf, nd = nf;
+      PixRec r;
+      r.lm = make_double2(ld, md);
+      r.nb = make_float4(__int_as_float(__double2loint(nd)), __int_as_float(__double2hiint(nd)), bf, nf - 1.0f);
+      r.f4 = make_float4(lf, mf, nf, bf);
+      px[p] = r;
+      const double nn = ld * ld + md * md + nd * nd;
+      bad |= !(fabs(nn - 1.0) <= 1e-5);
+      const double inv = 1.0 / sqrt(nn);
+      ux[k] = ld * inv; uy[k] = md * inv; uz[k] = nd * inv;
+      sum[0] += ux[k]; sum[1] += uy[k]; sum[2] += uz[k];
+    }
+    if (!sub && !tile) continue;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+    const bool wbad = __any_sync(0xffffffffu, bad);
+    __syncthreads();   // the previous tile's sums are read
+    if (lane == 0) {
+      for (int c = 0; c < 3; ++c) s_sum[warp][c] = sum[c];
+      s_bad[warp] = wbad;
+    }
+    __syncthreads();
+    double ax[2][3];
+    bool open[2];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {   // 0: sub-tile, 1: 1024-pixel tile
+      const int w = v ? 8 : sub_warps, w0 = warp & ~(w - 1);
+      double t[3] = {0.0, 0.0, 0.0};
+      open[v] = false;
+      for (int i = w0; i < w0 + w; ++i) {
+        for (int c = 0; c < 3; ++c) t[c] += s_sum[i][c];
+        open[v] |= s_bad[i] != 0;
+      }
+      const double nrm = sqrt(t[0] * t[0] + t[1] * t[1] + t[2] * t[2]);
+      double mind = 1.0;
+      for (int c = 0; c < 3; ++c) ax[v][c] = t[c] / nrm;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (base + 32 * k < npix) mind = fmin(mind, ax[v][0] * ux[k] + ax[v][1] * uy[k] + ax[v][2] * uz[k]);
+      for (int o = 16; o > 0; o >>= 1) mind = fmin(mind, __shfl_xor_sync(0xffffffffu, mind, o));
+      if (lane == 0) s_min[v][warp] = mind;
+    }
+    __syncthreads();
+    // lane 0: this warp's sub-tile, lane 1 of warp 0: the tile
+    const int v = lane == 1 ? 1 : 0;
+    const int w = v ? 8 : sub_warps;
+    const bool mine = v ? (tile && warp == 0) : (lane == 0 && sub && (warp & (sub_warps - 1)) == 0);
+    const int64_t first = (int64_t)sb * 1024 + (v ? 0 : warp * 128);
+    if (mine && first < npix) {
+      double mind = 1.0;
+      for (int i = warp; i < warp + w; ++i) mind = fmin(mind, s_min[v][i]);
+      const double alpha = open[v] ? 3.14159265358979323846 : acos(fmax(-1.0, fmin(1.0, mind))) + 1e-9;
+      ExactCone e;
+      e.cx = ax[v][0]; e.cy = ax[v][1]; e.cz = ax[v][2];
+      e.cos_a = cos(alpha);
+      e.sin_a = sin(alpha);
+      e.pad = 0.0;
+      (v ? tile : sub)[first / (v ? 1024 : 128 * sub_warps)] = e;
+    }
   }
 }
 
@@ -244,23 +336,6 @@ __global__ void k_mask(const float* __restrict__ l, const float* __restrict__ m,
     float c = occ_dot(l[p], m[p], n[p], x[e], y[e], z[e], invn[e]);
     float cp = cpe ? cpe[e] : cosphi;
     mask[i] = (c >= cp) ? 1 : 0;
-  }
-}
-
-// Stage-1 pixel records: (l, m) as FP64, (n as FP64 bits, B, nm1), (l, m, n, B).
-__global__ void k_pack_pixels(const float* __restrict__ B, const float* __restrict__ l,
-                              const float* __restrict__ m, const float* __restrict__ n,
-                              int64_t npix, PixRec* __restrict__ px) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += stride) {
-    float lf = l[i], mf = m[i], nf = n[i], bf = B[i];
-    PixRec r;
-    r.lm = make_double2((double)lf, (double)mf);
-    double nd = (double)nf;
-    r.nb = make_float4(__int_as_float(__double2loint(nd)), __int_as_float(__double2hiint(nd)),
-                       bf, nf - 1.0f);
-    r.f4 = make_float4(lf, mf, nf, bf);
-    px[i] = r;
   }
 }
 
@@ -446,10 +521,14 @@ static int launch_grid(int64_t n, int threads) {
 }
 
 // --- internal entry points used by the pipeline -----------------------------
-int geom_pack_pixels(const float* B, const float* l, const float* m, const float* n,
-                     int64_t npix, PixRec* px, cudaStream_t s) {
+// sub_pix: 128, 256 or 0 (no sub-tile cones); tile_cones (1024-pixel tiles), queue (four ints to clear): nullable.
+int geom_pack_cones(const float* B, const float* l, const float* m, const float* n, int64_t npix, PixRec* px,
+                    ExactCone* sub_cones, int sub_pix, ExactCone* tile_cones, int* queue, cudaStream_t s) {
   if (npix <= 0) return VB_OK;
-  k_pack_pixels<<<launch_grid(npix, 256), 256, 0, s>>>(B, l, m, n, npix, px);
+  const int nsuper = (int)ceil_div(npix, 1024);
+  const int grid = nsuper < sm_count() * 16 ? nsuper : sm_count() * 16;
+  k_pack_cones<<<grid, 256, 0, s>>>(B, l, m, n, npix, nsuper, px, sub_pix ? sub_cones : nullptr, sub_pix == 256 ? 2 : 1,
+                                    tile_cones, queue);
   VB_LAUNCH_CHECK();
   return VB_OK;
 }

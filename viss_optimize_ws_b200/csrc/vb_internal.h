@@ -42,8 +42,8 @@ struct __align__(16) PixRec {
   float4 nb;
   float4 f4;
 };
-int geom_pack_pixels(const float* B, const float* l, const float* m, const float* n, int64_t npix,
-                     PixRec* px, cudaStream_t s);
+int geom_pack_cones(const float* B, const float* l, const float* m, const float* n, int64_t npix, PixRec* px,
+                    ExactCone* sub_cones, int sub_pix, ExactCone* tile_cones, int* queue, cudaStream_t s);
 int geom_exact_cones(int tile_pix, const float* l, const float* m, const float* n, int64_t npix,
                      ExactCone* out, cudaStream_t s);
 int geom_validate_async(const float* u, const float* v, const float* w, int n_full, int nbl, int* d_bad,
@@ -59,6 +59,7 @@ struct Stage1Plan {
   int n_half, nbl;
   int nchunk, n_btile, n_items, grid;
   int ntile_cull;
+  int no_cones;       // VB_CULL_NONE: test every term at every pixel (no room or no use for cones)
   double max_turns;
   // track groups (vb_track.cu): 1 = the call plans them
   int track;
@@ -108,6 +109,7 @@ int track_group(const vb_baselines* bl, const Stage1Plan& p, const Stage1Buffers
 int track_sum(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s);
 
 int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts* o, Stage1Plan* p);
+size_t stage1_shrink(Stage1Plan* p, size_t cap);
 size_t stage1_carve(const Stage1Plan& p, void* ws, size_t cap, Stage1Buffers* b, bool pack_pixels);
 // pixels_ready: lm/nb/f4 (and cones for VB_CULL_EXACT) already hold this sky.
 // accumulate: V_half += this sky's sum (slabs of one sky) instead of V_half =.

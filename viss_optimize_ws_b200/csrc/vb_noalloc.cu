@@ -55,11 +55,7 @@ extern "C" int vb_viss_halfsym_noalloc(const vb_sky* sky, const vb_baselines* bl
   if (!bl->u || !bl->v || !bl->w) return fail(VB_ERR_INVALID, "vb_viss_halfsym_noalloc: u/v/w missing");
   if (p.blockage && (!bl->x1 || !bl->y1 || !bl->z1 || !bl->invn1 || !bl->x2 || !bl->y2 || !bl->z2 || !bl->invn2))
     return fail(VB_ERR_INVALID, "vb_viss_halfsym_noalloc: endpoint arrays missing");
-  size_t need = stage1_carve(p, nullptr, 0, nullptr, true);
-  if (p.track && need > (size_t)VB_VISS_NOALLOC_MAX_BYTES) {   // the per-term kernel alone needs less
-    p.track = 0;
-    need = stage1_carve(p, nullptr, 0, nullptr, true);
-  }
+  size_t need = stage1_shrink(&p, (size_t)VB_VISS_NOALLOC_MAX_BYTES);
   // Fit an automatic plan into the fixed scratch: fewer, larger pixel chunks
   // shrink the partial-sum buffer (results stay within FP32-sum rounding of
   // the default plan).  A chunk size the caller set is kept as given.

@@ -774,7 +774,7 @@ static int run_slabs(vb_pipeline* p, const float* B_host, int scale, float* C_ho
     Stage1Plan q{};
     VB_TRY(stage1_plan(&sky, &bl, &o1, &q));
     Stage1Buffers b;
-    if (q.track && !stage1_carve(q, p->ws1, p->ws1_bytes, &b, true)) q.track = 0;
+    stage1_shrink(&q, p->ws1_bytes);
     if (!stage1_carve(q, p->ws1, p->ws1_bytes, &b, true))
       return fail(VB_ERR_NOMEM, "slab %d: stage-1 workspace too small", k);
     b.err = p->slab_err;

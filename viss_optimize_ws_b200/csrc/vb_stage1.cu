@@ -41,8 +41,15 @@ constexpr int S1_THREADS = 256;
 // the per-pixel test (vb_stage1_opts.mask_visible_tiles).  A template value of
 // its own, so that the default tile-cone kernel carries no extra test.
 constexpr int kCullTileconeMV = 3;
+// And VB_CULL_NONE with occlusion: the terms that the per-pixel test includes,
+// found through exact cones on stages and sub-tiles of them.  The sums are the
+// same bit for bit (a hidden term adds a product with zero); testing every term
+// at every pixel ran at 0.47 of the SFU peak, this at 0.75 to 0.8.
+constexpr int kCullNoneExact = 4;
 template <int CULL>
 __host__ __device__ constexpr bool is_tilecone() { return CULL == VB_CULL_TILECONE || CULL == kCullTileconeMV; }
+template <int CULL>
+__host__ __device__ constexpr bool has_subtiles() { return is_tilecone<CULL>() || CULL == kCullNoneExact; }
 
 struct S1Args {
   const PixRec* __restrict__ px;   // stage-1 pixel records (interleaved, one per pixel)
@@ -110,7 +117,7 @@ __device__ __forceinline__ int tile_class(const S1Args& a, const Baseline& b, in
     cone_classify(cone_dot(b.ux1, b.uy1, b.uz1, cx, cy, cz), cA, sA, b.c1, vis1, hid1);
     cone_classify(cone_dot(b.ux2, b.uy2, b.uz2, cx, cy, cz), cA, sA, b.c2, vis2, hid2);
     return (hid1 || hid2) ? kClsHid : ((vis1 && vis2 && CULL != kCullTileconeMV) ? kClsVis : kClsMix);
-  } else if constexpr (CULL == VB_CULL_EXACT) {
+  } else if constexpr (CULL == VB_CULL_EXACT || CULL == kCullNoneExact) {
     return exact_tile_class(a.cones + tile_id, b.x1, b.y1, b.z1, b.i1, b.c1, b.x2, b.y2, b.z2, b.i2, b.c2);
   } else {
     return kClsMix;
@@ -272,6 +279,12 @@ __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
       int ih = btile * (S1_THREADS * BPT) + warp * (32 * BPT) + k * 32 + lane;
       if constexpr (LIST) ih = ih < a.count[1] ? a.list[ih] : a.n_half;
       load_baseline(a, ih, raw, b);
+      if constexpr (CULL == kCullNoneExact) {
+        // endpoint times invn off the unit sphere: its cone tests decide nothing
+        // (a NaN horizon; the per-pixel thresholds are set)
+        if (!(fabsf(b.ux1 * b.ux1 + b.uy1 * b.uy1 + b.uz1 * b.uz1 - 1.0f) <= 2e-3f)) b.c1 = NAN;
+        if (!(fabsf(b.ux2 * b.ux2 + b.uy2 * b.uy2 + b.uz2 * b.uz2 - 1.0f) <= 2e-3f)) b.c2 = NAN;
+      }
       const float uu = b.uf, vv = b.vf, ww = b.wf;
       if (MODE == VB_PREC_FP32_FP64PH && b.active &&
           (fabsf(uu) >= (float)kMaxUvwF32X || fabsf(vv) >= (float)kMaxUvwF32X ||
@@ -311,7 +324,7 @@ __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
       const bool warp_live = __any_sync(0xffffffffu, any_live);
       const bool warp_mix = __any_sync(0xffffffffu, any_mix);
       // mixed tiles refined into exact sub-tiles count their terms per sub-tile
-      const bool refine = is_tilecone<CULL>() && warp_mix && a.refine_pix > 0;
+      const bool refine = has_subtiles<CULL>() && warp_mix && a.refine_pix > 0;
       const int64_t tile_terms = (int64_t)nact * (t1 - t0);
       cnt_all += tile_terms;
       if (!warp_live) cnt_hid += tile_terms;
@@ -658,7 +671,7 @@ __global__ void __launch_bounds__(S1_THREADS) k_term_counts(const S1Args a, int 
 
 // The same without culling: one class for every term.
 __global__ void k_term_counts_plain(unsigned long long* counters, int which, unsigned long long terms, const int* count) {
-  if (count[0] == 0) return;
+  if (count && count[0] == 0) return;
   atomicAdd(&counters[which], terms);
   atomicAdd(&counters[3], terms);
 }
@@ -763,6 +776,7 @@ static void* stage1_kernel_cull(int bpt, int minb, int cull) {
   if (cull == VB_CULL_TILECONE) return stage1_kernel<MODE, VB_CULL_TILECONE, LIST>(bpt, minb);
   if (cull == kCullTileconeMV) return stage1_kernel<MODE, kCullTileconeMV, LIST>(bpt, minb);
   if (cull == VB_CULL_EXACT) return stage1_kernel<MODE, VB_CULL_EXACT, LIST>(bpt, minb);
+  if (cull == kCullNoneExact) return stage1_kernel<MODE, kCullNoneExact, LIST>(bpt, minb);
   return stage1_kernel<MODE, VB_CULL_NONE, LIST>(bpt, minb);
 }
 
@@ -781,6 +795,11 @@ static int occupancy(int mode, int bpt, int minb, int cull, size_t smem) {
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, S1_THREADS, smem) != cudaSuccess) return 1;
   return n < 1 ? 1 : n;
+}
+
+static int kernel_cull(const Stage1Plan& p) {
+  if (p.mask_visible) return kCullTileconeMV;
+  return p.cull == VB_CULL_NONE && p.blockage && !p.no_cones ? kCullNoneExact : p.cull;
 }
 
 static bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
@@ -807,6 +826,8 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
   q.npix = sky->npix;
   q.n_half = bl->n_full / 2;
   q.nbl = bl->nbl;
+  // below about 2e7 terms the cones cost as much as they save
+  q.no_cones = (double)q.n_half * (double)q.npix < 2e7;
 
   int stage = o->stage_pix > 0 ? o->stage_pix : 1024;
   if (!is_pow2(stage) || stage < 32 || stage > 2048)
@@ -840,11 +861,12 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
     if (!is_pow2(r) || r < 32) return fail(VB_ERR_INVALID, "stage 1: refine_pix=%d (power of two >= 32)", r);
     if (r < q.cull_tile && r <= q.stage_pix) q.refine_pix = r;
   }
+  if (kernel_cull(q) == kCullNoneExact && q.stage_pix > 128) q.refine_pix = 128;
 
   const int per_tile = S1_THREADS * q.bpt;
   q.n_btile = (int)ceil_div(q.n_half, per_tile);
   size_t smem = 2 * (size_t)stage * sizeof(PixRec);   // two staging buffers
-  int occ = occupancy(q.precision, q.bpt, q.minb, q.mask_visible ? kCullTileconeMV : q.cull, smem);
+  int occ = occupancy(q.precision, q.bpt, q.minb, kernel_cull(q), smem);
   int capacity = sm_count() * occ;
   q.grid = capacity;
   // enough items per CTA that the dynamic queue's tail (one item) stays short
@@ -880,7 +902,7 @@ size_t stage1_carve(const Stage1Plan& p, void* ws, size_t cap, Stage1Buffers* b,
   x.err = c.take<unsigned>(4);   // first: vb_workspace_error_flags reads it at offset 0
   if (pack_pixels) {
     x.px = c.take<PixRec>(p.npix);
-    if (p.cull == VB_CULL_EXACT) x.cones = c.take<ExactCone>(p.ntile_cull);
+    if (p.cull == VB_CULL_EXACT || kernel_cull(p) == kCullNoneExact) x.cones = c.take<ExactCone>(p.ntile_cull);
     if (p.refine_pix > 0) x.subcones = c.take<ExactCone>((size_t)ceil_div(p.npix, p.refine_pix));
   }
   const int rows = p.track ? std::max(p.nchunk, p.trk_nchunk) : p.nchunk;
@@ -893,10 +915,28 @@ size_t stage1_carve(const Stage1Plan& p, void* ws, size_t cap, Stage1Buffers* b,
 }
 
 int stage1_prepare_pixels(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cudaStream_t s) {
-  VB_TRY(geom_pack_pixels(sky->B, sky->l, sky->m, sky->n, p.npix, b.px, s));
-  if (p.cull == VB_CULL_EXACT) VB_TRY(geom_exact_cones(p.cull_tile, sky->l, sky->m, sky->n, p.npix, b.cones, s));
-  if (p.refine_pix > 0) VB_TRY(geom_exact_cones(p.refine_pix, sky->l, sky->m, sky->n, p.npix, b.subcones, s));
+  const bool sub_fits = p.refine_pix == 0 || p.refine_pix == 128 || p.refine_pix == 256;
+  ExactCone* tile = b.cones && p.cull_tile == 1024 ? b.cones : nullptr;
+  VB_TRY(geom_pack_cones(sky->B, sky->l, sky->m, sky->n, p.npix, b.px, b.subcones, sub_fits ? p.refine_pix : 0, tile, b.queue, s));
+  if (b.cones && !tile) VB_TRY(geom_exact_cones(p.cull_tile, sky->l, sky->m, sky->n, p.npix, b.cones, s));
+  if (!sub_fits) VB_TRY(geom_exact_cones(p.refine_pix, sky->l, sky->m, sky->n, p.npix, b.subcones, s));
   return track_prepare_pixels(sky, p, b, s);
+}
+
+// Turns the parts of a plan off that need scratch beyond the per-term kernel's
+// own, until it fits; returns the bytes it then needs.
+size_t stage1_shrink(Stage1Plan* p, size_t cap) {
+  size_t need = stage1_carve(*p, nullptr, 0, nullptr, true);
+  if (need > cap && p->track) {
+    p->track = 0;
+    need = stage1_carve(*p, nullptr, 0, nullptr, true);
+  }
+  if (need > cap && kernel_cull(*p) == kCullNoneExact) {
+    p->no_cones = 1;
+    p->refine_pix = 0;
+    need = stage1_carve(*p, nullptr, 0, nullptr, true);
+  }
+  return need;
 }
 
 int stage1_run(const vb_sky* sky, const vb_baselines* bl, const Stage1Plan& p, const Stage1Buffers& b,
@@ -920,11 +960,11 @@ int stage1_run(const vb_sky* sky, const vb_baselines* bl, const Stage1Plan& p, c
   a.cp1 = bl->cosphi1; a.cp2 = bl->cosphi2; a.cosphi = bl->cosphi;
   a.n_half = p.n_half; a.nbl = p.nbl; a.blockage = p.blockage; a.phase_corrected = p.phase_corrected;
   a.queue = b.queue; a.partial = b.partial; a.counters = counters; a.err = b.err;
-  const int kcull = p.mask_visible ? kCullTileconeMV : p.cull;
+  const int kcull = kernel_cull(p);
   const void* kern = stage1_kernel_of(p.precision, p.bpt, p.minb, kcull);
   const size_t smem = 2 * (size_t)p.stage_pix * sizeof(PixRec);
   VB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  VB_CUDA(cudaMemsetAsync(b.queue, 0, 4 * sizeof(int), s));
+  if (pixels_ready) VB_CUDA(cudaMemsetAsync(b.queue, 0, 4 * sizeof(int), s));   // (else the packing cleared it)
   if (p.track) {
     // The device decides: with factored groups the plain kernel's queue starts
     // past its last item and the list kernel runs, without any the other way
@@ -932,15 +972,17 @@ int stage1_run(const vb_sky* sky, const vb_baselines* bl, const Stage1Plan& p, c
     a.list = b.trk.direct;
     a.count = b.trk.count;
     VB_TRY(track_group(bl, p, b, s));
-    if (counters) {
-      if (p.cull == VB_CULL_NONE) {
-        k_term_counts_plain<<<1, 1, 0, s>>>(counters, p.blockage ? 1 : 0, (unsigned long long)p.n_half * p.npix,
-                                            b.trk.count);
-        VB_LAUNCH_CHECK();
-      } else {
-        VB_TRY(p.bpt == 1 ? term_counts<1>(a, p, s) : p.bpt == 2 ? term_counts<2>(a, p, s) : term_counts<4>(a, p, s));
-      }
+    if (counters && p.cull == VB_CULL_NONE && !p.blockage) {
+      k_term_counts_plain<<<1, 1, 0, s>>>(counters, 0, (unsigned long long)p.n_half * p.npix, b.trk.count);
+      VB_LAUNCH_CHECK();
+    } else if (counters && p.cull != VB_CULL_NONE) {
+      VB_TRY(p.bpt == 1 ? term_counts<1>(a, p, s) : p.bpt == 2 ? term_counts<2>(a, p, s) : term_counts<4>(a, p, s));
     }
+  }
+  if (counters && kcull == kCullNoneExact) {   // without culling every term counts as tested
+    k_term_counts_plain<<<1, 1, 0, s>>>(counters, 1, (unsigned long long)p.n_half * p.npix, nullptr);
+    VB_LAUNCH_CHECK();
+    a.counters = nullptr;
   }
   void* args[] = {&a};
   if (kbeg) VB_CUDA(record_event(kbeg, s));
@@ -994,11 +1036,7 @@ extern "C" int vb_viss_halfsym(const vb_sky* sky, const vb_baselines* bl, const 
   if (p.blockage && (!bl->x1 || !bl->y1 || !bl->z1 || !bl->invn1 || !bl->x2 || !bl->y2 || !bl->z2 || !bl->invn2))
     return fail(VB_ERR_INVALID, "vb_viss_halfsym: endpoint arrays missing");
   Stage1Buffers b;
-  size_t need = stage1_carve(p, nullptr, 0, nullptr, true);
-  if (p.track && ws_bytes < need) {   // the per-term kernel alone needs less
-    p.track = 0;
-    need = stage1_carve(p, nullptr, 0, nullptr, true);
-  }
+  const size_t need = stage1_shrink(&p, ws_bytes);
   if (!workspace || ws_bytes < need)
     return fail(VB_ERR_NOMEM, "vb_viss_halfsym: workspace %zu bytes < %zu", ws_bytes, need);
   if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
@@ -1050,8 +1088,7 @@ extern "C" int vb_stage1_tile_classes(const vb_sky* sky, const vb_baselines* bl,
     }
   }
   Stage1Buffers b;
-  p.track = 0;
-  size_t need = stage1_carve(p, nullptr, 0, nullptr, true);
+  const size_t need = stage1_shrink(&p, ws_bytes);
   if (!workspace || ws_bytes < need)
     return fail(VB_ERR_NOMEM, "vb_stage1_tile_classes: workspace %zu bytes < %zu", ws_bytes, need);
   if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0)
