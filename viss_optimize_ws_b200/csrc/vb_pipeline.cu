@@ -126,7 +126,7 @@ struct vb_pipeline {
   vb_seg_params* segp = nullptr;
   double* wsum = nullptr;
   unsigned long long* counters = nullptr;  // [0..3] stage 1, [4..7] stage 2
-  unsigned char* rep = nullptr;            // page-locked copies of what a report reads (see report_async)
+  unsigned char* rep = nullptr;            // holds the three above, so that a report reads one range (ReportWords)
   // timing / graph
   cudaEvent_t ev[10] = {};
   cudaStream_t s_side = nullptr;   // stage-2 grouping, concurrent with stage 1
@@ -171,15 +171,19 @@ extern "C" void vb_run_config_defaults(vb_run_config* c) {
   c->nm1_fast = 1;
 }
 
-// Host copies of the device words that a report holds: counters, group total,
-// error words, segment parameters (after these).  They are enqueued before the
-// call's one synchronisation; as synchronous copies after it they took 40 us of a
-// 360 us day.
+// What a report reads from the device, in one range there: counters, group total,
+// error words and (after these) the segment parameters.  One copy; as a copy each
+// after the run they took 40 us of a 360 us day.
 struct ReportWords {
   unsigned long long cnt[8];
-  double wsum;
-  unsigned e1, e2;
+  double wsum[2];
+  unsigned err[4];   // stage 1, stage 2
 };
+
+__global__ void k_report_errors(unsigned* out, const unsigned* e1, const unsigned* e2) {
+  out[0] = *e1;
+  out[1] = e2 ? *e2 : 0u;
+}
 
 template <class T>
 static int dalloc(vb_pipeline* p, T** ptr, size_t count) {
@@ -208,7 +212,6 @@ static void pipeline_free(vb_pipeline* p) {
   if (p->s_side) cudaStreamDestroy(p->s_side);
   if (p->orb) vb_orbit_destroy(p->orb);
   for (void* q : p->owned) cudaFree(q);
-  if (p->rep) cudaFreeHost(p->rep);
   if (p->s) cudaStreamDestroy(p->s);
   delete p;
 }
@@ -452,10 +455,10 @@ extern "C" int vb_pipeline_create(const vb_run_config* c, vb_pipeline** out) {
   PTRY(dalloc(p, &p->Vf, (size_t)2 * p->n_full));
   PTRY(dalloc(p, &p->C, p->nres));
   PTRY(dalloc(p, &p->W, p->nres));
-  PTRY(dalloc(p, &p->segp, p->nseg));
-  PTRY(dalloc(p, &p->wsum, 2));
-  PTRY(dalloc(p, &p->counters, 8));
-  PCUDA(cudaMallocHost(reinterpret_cast<void**>(&p->rep), sizeof(ReportWords) + (size_t)p->nseg * sizeof(vb_seg_params)));
+  PTRY(dalloc(p, &p->rep, sizeof(ReportWords) + (size_t)p->nseg * sizeof(vb_seg_params)));
+  p->counters = reinterpret_cast<ReportWords*>(p->rep)->cnt;
+  p->wsum = reinterpret_cast<ReportWords*>(p->rep)->wsum;
+  p->segp = reinterpret_cast<vb_seg_params*>(p->rep + sizeof(ReportWords));
   PCUDA(cudaMemsetAsync(p->counters, 0, 8 * sizeof(unsigned long long), p->s));
   PCUDA(cudaStreamSynchronize(p->s));
 #undef PTRY
@@ -634,21 +637,18 @@ static int plan_stages(vb_pipeline* p) {
   return VB_OK;
 }
 
-static int report_async(vb_pipeline* p, vb_report* r) {
-  if (!r) return VB_OK;
-  ReportWords* h = reinterpret_cast<ReportWords*>(p->rep);
-  h->e2 = 0;
-  VB_CUDA(cudaMemcpyAsync(h->cnt, p->counters, sizeof(h->cnt), cudaMemcpyDeviceToHost, p->s));
-  VB_CUDA(cudaMemcpyAsync(&h->wsum, p->wsum, sizeof(double), cudaMemcpyDeviceToHost, p->s));
-  VB_CUDA(cudaMemcpyAsync(&h->e1, p->b1.err, sizeof(unsigned), cudaMemcpyDeviceToHost, p->s));
-  if (p->ws2) VB_CUDA(cudaMemcpyAsync(&h->e2, p->ws2, sizeof(unsigned), cudaMemcpyDeviceToHost, p->s));   // stage-2 word: offset 0
-  VB_CUDA(cudaMemcpyAsync(p->rep + sizeof(ReportWords), p->segp, p->nseg * sizeof(vb_seg_params), cudaMemcpyDeviceToHost, p->s));
-  return VB_OK;
-}
-
-// After report_async and a synchronisation of p->s.
+// Ends a run: waits for the stream and fills the report.
 static int fill_report(vb_pipeline* p, vb_report* r) {
-  if (!r) return VB_OK;
+  if (!r) {
+    VB_CUDA(cudaStreamSynchronize(p->s));
+    return VB_OK;
+  }
+  std::vector<unsigned char> host(sizeof(ReportWords) + (size_t)p->nseg * sizeof(vb_seg_params));
+  k_report_errors<<<1, 1, 0, p->s>>>(reinterpret_cast<ReportWords*>(p->rep)->err, p->b1.err,
+                                     static_cast<const unsigned*>(p->ws2));   // stage-2 word: offset 0
+  VB_LAUNCH_CHECK();
+  VB_CUDA(cudaMemcpyAsync(host.data(), p->rep, host.size(), cudaMemcpyDeviceToHost, p->s));
+  VB_CUDA(cudaStreamSynchronize(p->s));
   std::memset(r, 0, sizeof(*r));
   r->npix_hi = (int)(p->npix >> 31);
   r->npix_lo = (int)(p->npix & 0x7fffffff);
@@ -666,19 +666,19 @@ static int fill_report(vb_pipeline* p, vb_report* r) {
   r->t_s2_kernel_ms = k2;
   r->graph_kernels = p->graph_kernels;
   r->bl_max_m = effective_bl_max(p);
-  const ReportWords* h = reinterpret_cast<const ReportWords*>(p->rep);
+  const ReportWords* h = reinterpret_cast<const ReportWords*>(host.data());
   for (int k = 0; k < 4; ++k) {
     r->s1_counters[k] = h->cnt[k];
     r->s2_counters[k] = h->cnt[4 + k];
   }
-  r->w_scalar_total = h->wsum;
-  const vb_seg_params* sp = reinterpret_cast<const vb_seg_params*>(p->rep + sizeof(ReportWords));
+  r->w_scalar_total = h->wsum[0];
+  const vb_seg_params* sp = reinterpret_cast<const vb_seg_params*>(host.data() + sizeof(ReportWords));
   long long g = 0;
   for (int k = 0; k < p->nseg; ++k) g += sp[k].nuniq;
   r->groups_total = g;
   r->stage1_terms = (long long)p->npix * p->n_half;
   r->stage2_terms = (long long)p->npix * g;
-  r->error_flags = (int)(h->e1 | h->e2);
+  r->error_flags = (int)(h->err[0] | h->err[1]);
   return VB_OK;
 }
 
@@ -743,8 +743,6 @@ extern "C" int vb_pipeline_run(vb_pipeline* p, vb_report* r) {
   VB_CUDA(cudaSetDevice(p->cfg.device));
   VB_TRY(ensure_ready(p));
   VB_TRY(run_once(p));
-  VB_TRY(report_async(p, r));
-  VB_CUDA(cudaStreamSynchronize(p->s));
   VB_TRY(fill_report(p, r));
   return VB_OK;
 }
@@ -835,8 +833,6 @@ static int run_slabs(vb_pipeline* p, const float* B_host, int scale, float* C_ho
   VB_CUDA(record_event(p->ev[6], p->s));
   VB_CUDA(record_event(p->ev[7], p->s));
   VB_CUDA(record_event(p->ev[8], p->s));
-  VB_TRY(report_async(p, r));
-  VB_CUDA(cudaStreamSynchronize(p->s));
   VB_TRY(fill_report(p, r));
   if (r) {
     float te = 0.f;
@@ -866,8 +862,6 @@ extern "C" int vb_pipeline_run_host(vb_pipeline* p, const float* B_host, int sca
   if (V_half_host)
     VB_CUDA(cudaMemcpyAsync(V_half_host, p->Vh, (size_t)2 * p->n_half * sizeof(float), cudaMemcpyDeviceToHost, p->s));
   VB_CUDA(record_event(p->ev[4], p->s));
-  VB_TRY(report_async(p, r));
-  VB_CUDA(cudaStreamSynchronize(p->s));
   VB_TRY(fill_report(p, r));
   if (r) {
     float te = 0.f;
