@@ -59,6 +59,7 @@ struct Stage1Plan {
   int n_half, nbl;
   int nchunk, n_btile, n_items, grid;
   int ntile_cull;
+  int whole_chunk;    // chunk_pix before a small call was split below its cull tile (0: not)
   int no_cones;       // VB_CULL_NONE: test every term at every pixel (no room or no use for cones)
   double max_turns;
   // track groups (vb_track.cu): 1 = the call plans them

@@ -885,6 +885,23 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
     chunk = o->chunk_pix;
   }
   if (chunk > INT32_MAX) chunk = (INT32_MAX / q.cull_tile) * (int64_t)q.cull_tile;
+  // A small call has fewer (baseline tile, cull tile) items than the chip has
+  // room for: items then take parts of a cull tile, halved until there are 4 for
+  // each resident CTA (their work differs with the horizon), but below 256
+  // pixels only while a CTA has none, since each repeats the baselines' set-up.
+  // Measured, whole tiles / 4 and 256 / 2 and 128 / 4 and 128 / 8 and 128 (one B200,
+  // 21 pairs): 1024-pixel tiles of nside 64, 100 steps: 172 / 123 / 123 / 129 / 130 us;
+  // 4096 of nside 128, 60 steps: 311 / 210 / 206 / 210 / 262; 16384 of nside 256, 60 steps:
+  // 1036 / 579 / 621 / 578 / 608; no blockage, nside 64, 64 steps: 77 / 78 / 92 / 91 / 92;
+  // 20 steps without culling, nside 64: 116 us whole, 79 at 256 pixels, 69 at 128.
+  if (o->chunk_pix == 0 && chunk == q.cull_tile) {
+    q.whole_chunk = (int)chunk;
+    for (;;) {
+      const int64_t have = ceil_div(q.npix, chunk) * q.n_btile;
+      if (!(chunk > 256 ? have < 4 * (int64_t)capacity : chunk > 128 && have < capacity)) break;
+      chunk /= 2;
+    }
+  }
   q.chunk_pix = (int)chunk;
   q.nchunk = (int)ceil_div(q.npix, q.chunk_pix);
   int64_t items = (int64_t)q.n_btile * q.nchunk;
@@ -934,6 +951,13 @@ size_t stage1_shrink(Stage1Plan* p, size_t cap) {
   if (need > cap && kernel_cull(*p) == kCullNoneExact) {
     p->no_cones = 1;
     p->refine_pix = 0;
+    need = stage1_carve(*p, nullptr, 0, nullptr, true);
+  }
+  if (need > cap && p->whole_chunk > p->chunk_pix) {
+    p->chunk_pix = p->whole_chunk;
+    p->nchunk = (int)ceil_div(p->npix, p->chunk_pix);
+    p->n_items = p->n_btile * p->nchunk;
+    if (p->grid > p->n_items) p->grid = p->n_items > 0 ? p->n_items : 1;
     need = stage1_carve(*p, nullptr, 0, nullptr, true);
   }
   return need;
