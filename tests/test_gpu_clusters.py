@@ -37,11 +37,11 @@ def setup(vb, nside, npix, lam, steps, day, earth=0):
 
 
 @pytest.mark.parametrize("nside,npix,lam,steps,day,earth,segs,mirror,blockage,cull", [
-    (256, 100003, 300.0, 500, 1, 0, 2, 1, 1, 2),     # ragged sky, uneven segments
-    (512, 262144, 30.0, 1000, 3, 0, 1, 1, 1, 2),     # long tracks: full clusters
-    (512, 131072, 300.0, 700, 8, 0, 3, 0, 1, 0),     # signed set, halves of clusters, no block culling
-    (256, 131072, 300.0, 300, 5, 0, 1, 0, 0, 0),     # group averages
-    (256, 131072, 300.0, 400, 1, 9, 2, 1, 1, 2),     # Earth orbits: few clusters or none
+    (512, 3000001, 300.0, 500, 1, 0, 2, 1, 1, 2),     # ragged sky, uneven segments
+    (512, 1200000, 30.0, 1000, 3, 0, 1, 1, 1, 2),     # long tracks: full clusters
+    (512, 800000, 300.0, 700, 8, 0, 3, 0, 1, 0),     # signed set, halves of clusters, no block culling
+    (512, 1800000, 300.0, 300, 5, 0, 1, 0, 0, 0),     # group averages
+    (512, 2200000, 300.0, 400, 1, 9, 2, 1, 1, 2),     # Earth orbits: few clusters or none
 ])
 def test_clusters_vs_fp64_reconstruction(vb, gpu, nside, npix, lam, steps, day, earth, segs, mirror, blockage, cull):
     sky, bl, V, keep = setup(vb, nside, npix, lam, steps, day, earth)
@@ -58,7 +58,7 @@ def test_clusters_vs_fp64_reconstruction(vb, gpu, nside, npix, lam, steps, day, 
 
 def test_one_infinite_visibility_stays_in_its_own_pixels(vb, gpu):
     """An infinite V makes exactly the pixels that see its group non-finite."""
-    sky, bl, V, keep = setup(vb, 512, 131072, 30.0, 1000, 3)
+    sky, bl, V, keep = setup(vb, 512, 1200000, 30.0, 1000, 3)
     V[5000] = np.inf
     dV = dev(V)
     kw = dict(mirror=1, blockage=1, cull=2, lam=30.0)
@@ -69,7 +69,7 @@ def test_one_infinite_visibility_stays_in_its_own_pixels(vb, gpu):
 
 def test_overlapping_segment_table(vb, gpu):
     """A segment table whose ranges overlap or run past the day gives what the FP64 build gives."""
-    sky, bl, V, keep = setup(vb, 256, 100003, 300.0, 500, 1)
+    sky, bl, V, keep = setup(vb, 512, 2000003, 300.0, 500, 1)
     dV = dev(V)
     kw = dict(mirror=1, blockage=1, cull=2, lam=300.0)
     for t0, tl in (([0, 200], [250, 300]),):

@@ -43,14 +43,14 @@ def setup(vb, nside, npix, lam, steps, day=5, earth=0, tile=256, B=None):
 
 
 @pytest.mark.parametrize("nside,npix,steps,lam,day,earth,tile,cull,blockage,corrected", [
-    (128, 196608, 400, 300.0, 1, 0, 256, "tilecone", 1, 1),      # whole sky, steps not a multiple of a group
-    (128, 196608, 384, 300.0, 1, 0, 64, "tilecone", 1, 1),       # the smallest cull tiles: 64-pixel blocks only
-    (256, 786432, 97, 300.0, 3, 0, 4096, "tilecone", 1, 0),      # one short group a pair, raw phase
-    (256, 500003, 257, 30.0, 2, 0, 1024, "exact", 1, 1),         # ragged sky, a group of one step
-    (256, 500003, 257, 30.0, 2, 0, 1024, "none", 1, 0),
-    (128, 196608, 400, 300.0, 8, 0, 256, "none", 0, 1),          # no occlusion
-    (256, 786432, 130, 300.0, 1, 7, 1024, "tilecone", 1, 1),     # Earth orbits: some groups factored, some left
-    (64, 49152, 1500, 300.0, 1, 0, 1024, "tilecone", 1, 1),      # coarse sky
+    (128, 196608, 1100, 300.0, 1, 0, 256, "tilecone", 1, 1),      # whole sky, steps not a multiple of a group
+    (128, 196608, 1152, 300.0, 1, 0, 64, "tilecone", 1, 1),       # the smallest cull tiles: 64-pixel blocks only
+    (512, 3145728, 97, 300.0, 3, 0, 4096, "tilecone", 1, 0),      # one short group a pair, raw phase
+    (256, 600007, 385, 30.0, 2, 0, 1024, "exact", 1, 1),         # ragged sky, a group of one step
+    (256, 600007, 385, 30.0, 2, 0, 1024, "none", 1, 0),
+    (128, 196608, 1100, 300.0, 8, 0, 256, "none", 0, 1),          # no occlusion
+    (256, 786432, 386, 300.0, 1, 7, 1024, "tilecone", 1, 1),     # Earth orbits: some groups factored, some left
+    (64, 49152, 4500, 300.0, 1, 0, 1024, "tilecone", 1, 1),      # coarse sky
 ])
 def test_track_groups_vs_fp64_sum(vb, gpu, nside, npix, steps, lam, day, earth, tile, cull, blockage, corrected):
     c = setup(vb, nside, npix, lam, steps, day, earth, tile)
@@ -68,7 +68,7 @@ def test_track_groups_vs_fp64_sum(vb, gpu, nside, npix, steps, lam, day, earth, 
 @pytest.mark.parametrize("cull", ["none", "tilecone", "exact"])
 def test_track_groups_include_the_masked_terms(vb, gpu, orc, cull):
     """u = v = w = 0 and B = 1: V is the number of included pixels of each baseline."""
-    nside, steps, tile = 128, 400, 256
+    nside, steps, tile = 128, 1100, 256
     c = setup(vb, nside, 196608, 300.0, steps, B=np.ones(196608, np.float32))
     nh = c["bl"].n_full // 2
     zero = zeros(c["bl"].n_full)
@@ -92,7 +92,7 @@ def test_track_groups_include_the_masked_terms(vb, gpu, orc, cull):
 
 def test_track_groups_leave_irregular_input_to_the_per_term_kernel(vb, gpu):
     """An infinite pixel, shuffled pixels and scattered baselines: what the plain sum gives."""
-    c = setup(vb, 128, 196608, 300.0, 400)
+    c = setup(vb, 128, 196608, 300.0, 1100)
     B = get(c["keep"][3])
     B[1234] = np.inf
     dB = dev(B)
@@ -107,7 +107,7 @@ def test_track_groups_leave_irregular_input_to_the_per_term_kernel(vb, gpu):
     V, _ = stage1(c["sky"], c["bl"], precision=vb.PREC_FP32_FP64PH, cull=0)
     V64, _ = stage1(c["sky"], c["bl"], precision=vb.PREC_FP64, cull=0)
     assert max(rel_err(V, V64)) <= TOL
-    c = setup(vb, 128, 196608, 300.0, 400)
+    c = setup(vb, 128, 196608, 300.0, 1100)
     rng = np.random.default_rng(2)
     uvw = [dev(rng.uniform(-300, 300, c["bl"].n_full).astype(np.float32)) for _ in range(3)]
     c["bl"].u, c["bl"].v, c["bl"].w = (a.ptr for a in uvw)
@@ -118,7 +118,7 @@ def test_track_groups_leave_irregular_input_to_the_per_term_kernel(vb, gpu):
 
 def test_workspace_of_the_per_term_kernel_still_serves(vb, gpu):
     """A workspace that only the per-term kernel fits in is accepted, as is the fixed-scratch entry."""
-    c = setup(vb, 128, 196608, 300.0, 400)
+    c = setup(vb, 128, 196608, 300.0, 1100)
     o = vb.Stage1Opts(precision=vb.PREC_FP32_FP64PH, cull=1, phase_corrected=1, blockage=1)
     sky, bl = c["sky"], c["bl"]
     need = vb.lib().vb_stage1_workspace_bytes(C.byref(sky), C.byref(bl), C.byref(o))

@@ -76,7 +76,8 @@ struct TrackSub {
   float e[9], gamma, kappa, pad;
 };
 struct TrackPlan {
-  int mode, pad;
+  int mode;
+  float cost;         // cycles for each 32 terms, of kTermCycles on the per-term kernel
   TrackSub sub[4];
 };
 // One block of 64, 256 or 1024 pixels: centre and sine of the cone's half-angle,

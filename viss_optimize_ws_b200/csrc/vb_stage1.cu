@@ -515,6 +515,8 @@ __global__ void __maxnreg__(MINB == 3 ? 80 : 120) k_stage1(const S1Args a) {
   }
   __syncthreads();
   if (a.counters && threadIdx.x < 4) atomicAdd(&a.counters[threadIdx.x], s_cnt[threadIdx.x]);
+  // launched beside k_track_sum's last warps: what follows needs both kernels' sums
+  if constexpr (LIST) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Term counters of a call whose sum is factored: the classes and the warps of
@@ -1018,7 +1020,20 @@ int stage1_run(const vb_sky* sky, const vb_baselines* bl, const Stage1Plan& p, c
     const void* lk = stage1_kernel_cull<VB_PREC_FP32_FP64PH, true>(p.bpt, p.minb, kcull);
     VB_CUDA(cudaFuncSetAttribute(lk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void* largs[] = {&la};
-    VB_CUDA(cudaLaunchKernel(lk, dim3(p.grid), dim3(S1_THREADS), largs, smem, s));
+    // The two sums are independent.  k_track_sum's items differ by an order of
+    // magnitude (a warp whose pixels lie on the horizon), and its last ones leave
+    // most SMs idle: the list kernel's CTAs start as its CTAs end, and end after it.
+    cudaLaunchAttribute beside{};
+    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    beside.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc{};
+    lc.gridDim = dim3(p.grid);
+    lc.blockDim = dim3(S1_THREADS);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = s;
+    lc.attrs = &beside;
+    lc.numAttrs = 1;
+    VB_CUDA(cudaLaunchKernelExC(&lc, lk, largs));
   }
   VB_CUDA(cudaLaunchKernel(kern, dim3(p.grid), dim3(S1_THREADS), args, smem, s));
   if (kend) VB_CUDA(record_event(kend, s));

@@ -765,6 +765,7 @@ __global__ void __launch_bounds__(S2_THREADS, 2) k_recon_rec(const ReconArgs a) 
     atomicAdd(&a.counters[2], c_hid);
     atomicAdd(&a.counters[3], c_all);
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // launched beside k_recon_track: what follows needs both sums
 }
 
 // occ_mode 0 / 1 / other: per pixel, the visible ones of the group's members (all
@@ -1162,22 +1163,32 @@ size_t stage2_workspace(const Stage2Plan& p, void* ws, size_t cap, void** slices
 }
 
 template <class K>
-static int launch_persistent(K kern, const ReconArgs& a, cudaStream_t s) {
+static int launch_persistent(K kern, const ReconArgs& a, bool beside, cudaStream_t s) {
   int occ = 0;
   VB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, S2_THREADS, 0));
   if (occ < 1) occ = 1;
-  kern<<<sm_count() * occ, S2_THREADS, 0, s>>>(a);
-  VB_LAUNCH_CHECK();
+  // beside: k_recon_track runs before on this stream; the sums are independent, so
+  // the CTAs start as its CTAs end (and end after it, see the kernel's last line)
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t lc{};
+  lc.gridDim = dim3(sm_count() * occ);
+  lc.blockDim = dim3(S2_THREADS);
+  lc.stream = s;
+  lc.attrs = &attr;
+  lc.numAttrs = beside ? 1 : 0;
+  VB_CUDA(cudaLaunchKernelEx(&lc, kern, a));
   return VB_OK;
 }
 
 template <int MODE>
-static int launch_recon(const ReconArgs& a, bool members, int ppt, cudaStream_t s) {
-  if (members) return launch_persistent(k_recon_members<MODE>, a, s);
+static int launch_recon(const ReconArgs& a, bool members, int ppt, bool beside, cudaStream_t s) {
+  if (members) return launch_persistent(k_recon_members<MODE>, a, false, s);
   switch (ppt) {
-    case 1: return launch_persistent(k_recon_rec<MODE, 1>, a, s);
-    case 4: return launch_persistent(k_recon_rec<MODE, 4>, a, s);
-    default: return launch_persistent(k_recon_rec<MODE, 2>, a, s);
+    case 1: return launch_persistent(k_recon_rec<MODE, 1>, a, beside, s);
+    case 4: return launch_persistent(k_recon_rec<MODE, 4>, a, beside, s);
+    default: return launch_persistent(k_recon_rec<MODE, 2>, a, beside, s);
   }
 }
 
@@ -1309,10 +1320,10 @@ int stage2_finish(const vb_sky* sky, const vb_baselines* bl, const float* V_half
       VB_TRY(cluster_sum(sky, p, x.trk, x.sp, x.rec, x.ngroups, x.queue + 1, x.Cpart + (size_t)p.nchunk_target * (size_t)p.npix,
                          x.Wpart + (size_t)p.nchunk_target * (size_t)p.npix, st));
     switch (p.precision) {
-      case VB_PREC_REF32: VB_TRY(launch_recon<VB_PREC_REF32>(ra, members, p.ppt, st)); break;
-      case VB_PREC_FP64: VB_TRY(launch_recon<VB_PREC_FP64>(ra, members, p.ppt, st)); break;
-      case VB_PREC_FP32_FP64PH: VB_TRY(launch_recon<VB_PREC_FP32_FP64PH>(ra, members, p.ppt, st)); break;
-      default: VB_TRY(launch_recon<VB_PREC_FP32_DSPH>(ra, members, p.ppt, st)); break;
+      case VB_PREC_REF32: VB_TRY(launch_recon<VB_PREC_REF32>(ra, members, p.ppt, p.trk != 0, st)); break;
+      case VB_PREC_FP64: VB_TRY(launch_recon<VB_PREC_FP64>(ra, members, p.ppt, p.trk != 0, st)); break;
+      case VB_PREC_FP32_FP64PH: VB_TRY(launch_recon<VB_PREC_FP32_FP64PH>(ra, members, p.ppt, p.trk != 0, st)); break;
+      default: VB_TRY(launch_recon<VB_PREC_FP32_DSPH>(ra, members, p.ppt, p.trk != 0, st)); break;
     }
     if (kend) VB_CUDA(record_event(kend, st));
   } else if (kbeg) {

@@ -363,6 +363,7 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
     }
   }
   int mode = -1;
+  float best = 0.f;
   double uc[3];
   float e[9], R[4], gamma, kappa;
   if (__all_sync(0xffffffffu, fine)) {
@@ -385,7 +386,7 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
       turn = sqrtf(dx * dx + dy * dy + dz * dz) / (float)max(nv - 1, 1);   // a step
     }
     const float r64 = __uint_as_float(a.rmax[0]);
-    float best = 10.f;
+    best = 10.f;
     for (int ls = 0; ls <= 2; ++ls) {
       const int ks = 1 << ls;
       float M[4] = {0.f, 0.f, 0.f, 0.f};
@@ -429,7 +430,10 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
       }
     }
   }
-  if (lane == 0) a.plan[g].mode = mode;
+  if (lane == 0) {
+    a.plan[g].mode = mode;
+    a.plan[g].cost = best;
+  }
 }
 
 // Exclusive scans over the groups in (step block, pair) order, one CTA: place of
@@ -437,12 +441,32 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
 // before each group.  That list keeps the callers' order (steps, then pairs):
 // with a pair's consecutive steps side by side instead, a warp's baselines span
 // 32 steps of horizon motion and the per-term kernel ran up to 15 % slower.
-__global__ void __launch_bounds__(1024) k_track_scan(const TrackPlan* plan, int ngroups, int nbl, int gpp, int steps, int* off,
+constexpr float kTermCycles = 18.f;   // k_stage1, a warp's cycles for each 32 terms
+
+__global__ void __launch_bounds__(1024) k_track_scan(TrackPlan* plan, int ngroups, int nbl, int gpp, int steps, int* off,
                                                      int* left, int* count, int* queue) {
   __shared__ unsigned long long s_w[32];
   __shared__ unsigned long long s_base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // What the factored groups are expected to save, of the whole call.  Below 8 %
+  // none is factored: the baselines left fill the per-term kernel's warps less well
+  // (their horizons differ more) and there are two tails; calls of 2e9 to 8e9 terms
+  // with 2 to 6 % expected ran 1 to 8 % slower than without.
+  float save = 0.f;
+  for (int s = threadIdx.x; s < ngroups; s += 1024) {
+    const int j = s / nbl;
+    const TrackPlan& t = plan[(s - j * nbl) * gpp + j];
+    if (t.mode >= 0) save += (kTermCycles - t.cost) / kTermCycles * (float)min(TK_GROUP, steps - j * TK_GROUP);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) save += __shfl_xor_sync(0xffffffffu, save, o);
+  if (lane == 0) s_w[warp] = (unsigned long long)__float_as_uint(save);
   if (threadIdx.x == 0) s_base = 0ull;
+  __syncthreads();
+  save = 0.f;
+  for (int w = 0; w < 32; ++w) save += __uint_as_float((unsigned)s_w[w]);
+  if (!(save >= 0.08f * (float)steps * (float)nbl))
+    for (int s = threadIdx.x; s < ngroups; s += 1024) plan[s].mode = -1;
   __syncthreads();
   for (int g0 = 0; g0 < ngroups; g0 += 1024) {
     const int s = g0 + threadIdx.x;
@@ -852,6 +876,7 @@ __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_consta
   TrackSmem& sm = *reinterpret_cast<TrackSmem*>(smem_raw);
   const int lane = threadIdx.x & 31;
   TrackWarp& w = sm.w[threadIdx.x >> 5];
+  asm volatile("griddepcontrol.launch_dependents;");   // the list kernel may take SMs that this one leaves
   const int nfast = a.count[0];
   const int n_items = nfast * a.nchunk;
   for (int i = threadIdx.x; i < TK_SETS * 2 * TK_JMAX; i += TK_THREADS) {
@@ -997,13 +1022,16 @@ static void set_tables(float* scale, unsigned char* dest) {
 }
 
 // Track groups are in use for the FP32 sum with FP64 phase where the call is
-// large enough that the planning launches (about 20 us) do not count, and
-// where groups and pixel blocks exist: 96 steps (a group of 128 mostly filled),
-// 2e9 terms (about 2 ms on the per-term kernel), cull tiles of 64 pixels or more.
+// large enough that the planning launches and a second tail (40 to 60 us) do not
+// count, and where groups and pixel blocks exist: 96 steps (a group of 128 mostly
+// filled), 6e9 terms (3 ms on the per-term kernel), cull tiles of 64 pixels or more.
+// One B200, 28 pairs, without / with: 4.4e9 terms (nside 256, 200 steps): lunar, 300 m
+// 2.21 / 1.34 ms, 30 m 2.20 / 1.58, Earth orbits, 300 m 2.10 / 2.16; 8.8e9 (400 steps):
+// 4.23 / 1.98, 4.17 / 2.40 and 4.03 / 3.92; nothing to factor, 8.3e9: 3.93 / 3.95.
 void track_plan(Stage1Plan* p, int items_per_cta) {
   p->track = 0;
   const int steps = p->n_half / p->nbl;
-  if (p->precision != VB_PREC_FP32_FP64PH || steps < 96 || (double)p->n_half * (double)p->npix < 2e9) return;
+  if (p->precision != VB_PREC_FP32_FP64PH || steps < 96 || (double)p->n_half * (double)p->npix < 6e9) return;
   int level = TK_LEVELS - 1;
   if (p->cull == VB_CULL_TILECONE) {
     if (p->cull_tile < tk_block(0)) return;

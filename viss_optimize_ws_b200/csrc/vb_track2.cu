@@ -250,11 +250,18 @@ __global__ void __launch_bounds__(1024) k_cluster_scan(const ClusterArgs a) {
       a.table[e].base = (int)(ex & 0xffffffffull);
     }
   }
-  const int nc = (int)(s_base >> 32);
+  int nc = (int)(s_base >> 32);
+  const int ng = *a.ngroups;
+  // Fewer than a quarter of the groups: what they save does not pay for the second
+  // kernel's tail (30 m, Earth orbits, nside 256 and 512: 1 to 3 % slower with them).
+  if (4 * (s_base & 0xffffffffull) < (unsigned long long)ng) {
+    nc = 0;
+    for (int e = threadIdx.x; e < 2 * a.entries; e += 1024) a.table[e].set = -1;
+    for (int g = threadIdx.x; g < ng; g += 1024) a.dst[g] = 0;
+  }
   __syncthreads();
   if (threadIdx.x == 0) s_base = 0ull;
   __syncthreads();
-  const int ng = *a.ngroups;
   for (int g0 = 0; g0 < ng; g0 += 1024) {
     const int g = g0 + threadIdx.x;
     const bool left = g < ng && a.dst[g] >= 0;
@@ -392,6 +399,7 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
   __shared__ unsigned char s_dest[G2_SETS][2 * G2_J];
   __shared__ int s_item;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  asm volatile("griddepcontrol.launch_dependents;");   // k_recon_rec may take SMs that this one leaves
   const int nc = a.count[0], nd = a.count[1];
   if (nc == 0) return;
   for (int i = threadIdx.x; i < G2_SETS * 2 * G2_J; i += G2_THREADS) {
@@ -629,16 +637,18 @@ static void poly_tables(float* scale, unsigned char* dest) {
 }
 
 // Clusters are in use for the FP32 sum with FP64 phase over representatives or
-// averages where the call is large enough for the planning launches (about
-// 30 us; 2e9 (baseline, pixel) pairs are about 0.3 ms of k_recon_rec) and where
-// a track can fill one (64 steps a segment on average).
+// averages where the call is large enough for the planning launches and a second
+// kernel's tail (3e10 (baseline, pixel) pairs, 2 ms of k_recon_rec; 8 pairs of
+// satellites, nside 256, one B200, without / with clusters: 400 steps, 9e9: 0.64 / 0.74 ms;
+// 1000 steps, 2e10: 1.32 / 1.35; 2000, 4e10: 2.48 / 2.30; nside 512, 400, 4e10: 1.87 /
+// 1.39) and where a track can fill one (64 steps a segment on average).
 void cluster_plan(Stage2Plan* p, int nbl) {
   p->trk = 0;
   const bool members = p->blockage && p->occ_mode != 2;
   if (p->precision != VB_PREC_FP32_FP64PH || members || nbl <= 0 || p->n_half_total % nbl != 0) return;
   const int64_t steps = p->n_half_total / nbl;
   const int64_t ntrk = p->mirror ? nbl : 2 * (int64_t)nbl;
-  if (ntrk > G2_TRACKS || steps < 64LL * p->nseg || (double)p->n_keyed_total * (double)p->npix < 2e9) return;
+  if (ntrk > G2_TRACKS || steps < 64LL * p->nseg || (double)p->n_keyed_total * (double)p->npix < 3e10) return;
   const int64_t entries = ntrk * (steps / 32 + p->nseg);
   if (entries > INT32_MAX / 64) return;
   p->trk_ntrk = (int)ntrk;
