@@ -69,7 +69,8 @@ int vb_workspace_error_flags(const void* workspace, unsigned* flags, void* strea
 #define VB_PREC_FP32_DSPH    3  /* phase as an exact double-single FP32 product; FP32 sincos; Kahan sums */
 
 /* Stage-1 culling semantics. */
-#define VB_CULL_NONE         0  /* per-pixel occlusion mask on every term (upstream plain kernel) */
+#define VB_CULL_NONE         0  /* per-pixel occlusion mask on every term (upstream plain kernel); blocks proven
+                                   all-visible / all-hidden skip the test, every term counts as masked */
 #define VB_CULL_TILECONE     1  /* upstream tile-cone semantics: hidden tiles skipped, all-visible tiles summed
                                    WITHOUT the per-pixel mask, mixed tiles masked per pixel */
 #define VB_CULL_EXACT        2  /* same terms as VB_CULL_NONE; tiles proven all-visible / all-hidden with a
@@ -223,7 +224,9 @@ size_t vb_stage1_workspace_bytes(const vb_sky* sky, const vb_baselines* bl,
 /* V_half[2*ih+{0,1}] = (re, im) for half-baseline ih, ih in [0, n_full/2),
  * with upstream index map ih -> (ih/nbl)*2*nbl + ih%nbl
  * (common.hpp:213-220).  term_counters (nullable, device, 4 x uint64) are
- * incremented by the terms evaluated as [visible-fast, masked, hidden-skipped, total].
+ * incremented by the terms evaluated as [visible-fast, masked, hidden-skipped, total]:
+ * the terms that the per-term kernel takes on each path, also where consecutive steps
+ * of a pair are summed together (their sum holds the same terms).
  * Replaces viss_partial_all_halfsym<256,true> (viss_recon_kernel.cuh:200-287)
  * and viss_partial_all_halfsym_tilecone<TILE,true>
  * (viss_recon_kernel_mirror_tile_vissfast.cuh:437-561). */

@@ -13,7 +13,8 @@
 // as warp-broadcasts.  Per pixel tile each warp takes one of three paths
 // (skip / unmasked / masked) from its lanes' tile classes, so the hot loop is
 // warp-uniform.  Partial sums per chunk are reduced in a fixed order
-// (deterministic).
+// (deterministic).  Large calls whose baselines form tracks (consecutive steps of
+// a pair) sum those in groups (vb_track.cu); this kernel takes the baselines left.
 //
 // Precision modes (the `MODE` template argument):
 //   REF32  : FP32 phase (upstream arithmetic), FP32 sincos, FP32 stage sums.
