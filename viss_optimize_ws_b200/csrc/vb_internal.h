@@ -138,7 +138,7 @@ struct Stage2Plan {
 struct GroupCluster;
 struct GroupRec;
 struct ClusterBuffers {
-  int *count = nullptr, *slots = nullptr, *order = nullptr, *dst = nullptr, *list = nullptr;
+  int *count = nullptr, *steps = nullptr, *slots = nullptr, *order = nullptr, *dst = nullptr, *list = nullptr;
   GroupCluster *table = nullptr, *clu = nullptr;
   vb_seg_params* spd = nullptr;
   unsigned* rmax = nullptr;

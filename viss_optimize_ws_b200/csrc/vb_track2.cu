@@ -27,6 +27,7 @@
 #include "vb_common.cuh"
 #include "vb_geom.cuh"
 #include "vb_internal.h"
+#include "vb_segments.h"
 #include "vb_stage1.cuh"
 #include "vb_stage2.cuh"
 #include "vb_track.cuh"
@@ -68,6 +69,7 @@ struct ClusterArgs {
   const int *seg_t0, *seg_tlen;
   int ntrk, nseg, n_keyed, entries;
   const unsigned* rmax;
+  int* steps;                                // of each segment (segment_steps)
   int *slots, *order, *dst, *list, *count;   // count: clusters, groups left to k_recon_rec
   GroupCluster *table, *clu;                 // by entry; those in use, in a row
   vb_seg_params* spd;
@@ -75,10 +77,26 @@ struct ClusterArgs {
 constexpr int kClusterWords = sizeof(GroupCluster) / sizeof(int);
 static_assert(kClusterWords == 16, "a lane copies one word of a cluster");
 
-// Steps of a segment that the slots hold (none for a table that runs past the baselines).
-__device__ __forceinline__ int seg_steps(const ClusterArgs& a, int seg) {
-  const int t0 = a.seg_t0[seg], tl = a.seg_tlen[seg];
-  return t0 >= 0 && tl > 0 && (int64_t)a.ntrk * ((int64_t)t0 + tl) <= a.n_keyed ? tl : 0;
+// Steps of each segment that its slots hold, one warp from the last segment back:
+// slots, track orders and table entries of a segment are laid out by them, so two
+// segments must not share a step.
+__global__ void __launch_bounds__(32) k_cluster_steps(const ClusterArgs a) {
+  const int lane = threadIdx.x;
+  const int64_t steps = a.n_keyed / a.ntrk;
+  int after = INT32_MAX;   // smallest t0 of the segments past this pass
+  for (int top = a.nseg - 1; top >= 0; top -= 32) {
+    const int seg = top - lane;
+    const int t0 = seg >= 0 ? a.seg_t0[seg] : INT32_MAX;
+    int low = t0;          // smallest t0 from this segment on
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, low, o);
+      if (lane >= o) low = min(low, v);
+    }
+    const int prev = __shfl_up_sync(0xffffffffu, low, 1);
+    if (seg >= 0) a.steps[seg] = segment_steps(t0, a.seg_tlen[seg], lane ? min(after, prev) : after, steps);
+    after = min(after, __shfl_sync(0xffffffffu, low, 31));
+  }
 }
 
 // Each group's place on its representative's track: slots[segment][track][step].
@@ -91,7 +109,7 @@ __global__ void k_cluster_mark(const ClusterArgs a) {
     if ((unsigned)ck == 0u) continue;   // off the grid
     const int seg = (int)(ck >> 32), rep = a.svals[s0 + (L >> 1)];
     const int step = rep / a.ntrk, track = rep - step * a.ntrk;
-    const int t0 = a.seg_t0[seg], tl = seg_steps(a, seg);
+    const int t0 = a.seg_t0[seg], tl = a.steps[seg];
     if (step < t0 || step >= t0 + tl) continue;
     a.slots[(int64_t)a.ntrk * t0 + (int64_t)track * tl + (step - t0)] = g;
   }
@@ -102,7 +120,7 @@ __global__ void k_cluster_mark(const ClusterArgs a) {
 __global__ void __launch_bounds__(1024) k_cluster_cut(const ClusterArgs a) {
   __shared__ int s_m[G2_TRACKS], s_pre[G2_TRACKS];
   const int seg = blockIdx.x, lane = threadIdx.x & 31;
-  const int t0 = a.seg_t0[seg], tl = seg_steps(a, seg);
+  const int t0 = a.seg_t0[seg], tl = a.steps[seg];
   const int64_t base = (int64_t)a.ntrk * t0;
   for (int t = threadIdx.x >> 5; t < a.ntrk; t += 32) {
     const int64_t row = base + (int64_t)t * tl;
@@ -137,8 +155,7 @@ __global__ void __launch_bounds__(1024) k_cluster_cut(const ClusterArgs a) {
     if (m < G2_MIN) continue;
     const int k = (m + 31) / 32, size = (m + k - 1) / k;
     for (int c = 0; c < k; ++c) {
-      // region of the segment: ntrk clusters for every 32 steps before it and one more per segment
-      const int e = a.ntrk * (t0 / 32 + seg) + s_pre[t] + c;
+      const int64_t e = segment_entries(t0, seg, a.ntrk) + s_pre[t] + c;
       if (e >= a.entries) break;
       GroupCluster& q = a.table[2 * e];
       q.first = (int)(base + (int64_t)t * tl) + c * size;
@@ -662,6 +679,7 @@ void cluster_carve(const Stage2Plan& p, Carve& c, ClusterBuffers& x) {
   if (!p.trk) return;
   const size_t n = (size_t)p.n_keyed_total;
   x.count = c.take<int>(4);
+  x.steps = c.take<int>(p.nseg);
   x.slots = c.take<int>(n);
   x.order = c.take<int>(n);
   x.dst = c.take<int>(n);
@@ -680,11 +698,13 @@ int cluster_group(const Stage2Plan& p, const ClusterBuffers& x, const unsigned l
   a.skeys = skeys; a.svals = svals; a.start = start; a.ngroups = ngroups; a.sp = sp;
   a.seg_t0 = seg_t0; a.seg_tlen = seg_tlen;
   a.n_keyed = p.n_keyed_total; a.ntrk = p.trk_ntrk; a.nseg = p.nseg; a.entries = p.trk_entries;
-  a.rmax = x.rmax; a.slots = x.slots; a.order = x.order; a.dst = x.dst; a.list = x.list; a.count = x.count; a.table = x.table; a.clu = x.clu;
+  a.rmax = x.rmax; a.steps = x.steps; a.slots = x.slots; a.order = x.order; a.dst = x.dst; a.list = x.list; a.count = x.count; a.table = x.table; a.clu = x.clu;
   a.spd = x.spd;
   VB_CUDA(cudaMemsetAsync(x.slots, 0xff, (size_t)p.n_keyed_total * sizeof(int), s));
   VB_CUDA(cudaMemsetAsync(x.table, 0, 2 * (size_t)p.trk_entries * sizeof(GroupCluster), s));
   const int g = (int)std::min<int64_t>(ceil_div(p.n_keyed_total, 256), (int64_t)sm_count() * 16);
+  k_cluster_steps<<<1, 32, 0, s>>>(a);
+  VB_LAUNCH_CHECK();
   k_cluster_mark<<<g, 256, 0, s>>>(a);
   VB_LAUNCH_CHECK();
   k_cluster_cut<<<p.nseg, 1024, 0, s>>>(a);
