@@ -84,9 +84,14 @@ struct TrackArgs {
 // Pixel blocks: centre (mean of the pixel vectors), cone, and the largest
 // centre-pixel distance of the sky per level.  A value that is not finite, a
 // pixel vector off the unit sphere or an absurdly large brightness anywhere
-// makes the distances infinite, which keeps every group on the per-term kernel.  One CTA per 1024 pixels, 4 pixels per thread, so that a
-// half-warp holds a 64-pixel block and a pair of warps a 256-pixel block.
+// makes the distances infinite, which keeps every group on the per-term kernel.
+// Blocks of coincident pixels have no extent: the distances stay at kMinRadius or
+// above (what reads them divides by them).  One CTA per 1024 pixels, 4 pixels per
+// thread, so that a half-warp holds a 64-pixel block and a pair of warps a
+// 256-pixel block.
 // Bound: HBM (16 bytes read per pixel).
+constexpr float kMinRadius = 1e-6f;   // well under the extent of any block of distinct pixels
+
 struct BlockArgs {
   const float *B, *l, *m, *n;
   int64_t npix;
@@ -189,7 +194,7 @@ __global__ void __launch_bounds__(256) k_track_blocks(const BlockArgs a) {
         e.cen = make_float4(cc[lev][0], cc[lev][1], cc[lev][2], (float)sin(alpha));
         e.axis = make_float4((float)ax[lev][0], (float)ax[lev][1], (float)ax[lev][2], (float)cos(alpha));
         a.node[lev][blk] = e;
-        atomicMax(&a.rmax[lev], any_bad || !(r < 16.f) ? __float_as_uint(INFINITY) : __float_as_uint(r));
+        atomicMax(&a.rmax[lev], __float_as_uint(any_bad || !(r < 16.f) ? INFINITY : fmaxf(r, kMinRadius)));
       }
     }
     __syncthreads();
