@@ -1,0 +1,63 @@
+"""Factored sums with one term that matters: a sky of one source (stage 1).  Errors then
+cannot cancel, so this is the largest error of a term.
+
+The pairs move along tracks of one direction at 56 speeds, so that every polynomial is met
+at the ends of its range, and the source is the pixel that lies farthest along the tracks
+from its block's centre.
+
+Tolerance for |exp(i phi)|: half a step of the 2^-23-turn phase grid 3.7e-7, the angle in
+float32 2.4e-7 and its fl(2 pi) 1.7e-7, the SFU's sine and cosine 6e-7, polynomials
+6e-7 and their float sums 5e-7 (powers up to 2.5^n / n!), 2.5e-6 in all; the
+per-term kernel's own bound, with three roundings of the phase, is 2.1e-6.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from gpu_util import dev, geometry, sky_struct, stage1
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2.5e-6
+
+
+def tracks(vb, steps, speeds, axis, across, bend):
+    """Signed baselines of len(speeds) pairs: straight tracks with a bend of `bend` radians over 128 steps."""
+    n = len(speeds)
+    k = np.arange(steps)[:, None] - 0.5 * steps
+    s = np.asarray(speeds)[None, :] * k
+    c = s * (bend / 128) * k * 0.5
+    start = np.stack([np.linspace(-300, 250, n), np.linspace(200, 330, n), np.linspace(30, -90, n)], 1)
+    u = start[None] + s[:, :, None] * axis + c[:, :, None] * across
+    full = np.concatenate([-u, u], 1).reshape(-1, 3).astype(np.float32)
+    bl = vb.Baselines(n_full=full.shape[0], nbl=n)
+    d = {key: dev(np.ascontiguousarray(full[:, i])) for i, key in enumerate("uvw")}
+    for key, b in d.items():
+        setattr(bl, key, b.ptr)
+    return bl, d
+
+
+@pytest.mark.parametrize("nside,bend", [(512, 0.0), (512, 0.05), (512, 0.2), (256, 0.4), (128, 0.05)])
+def test_one_source(vb, gpu, nside, bend):
+    npix = min(12 * nside * nside, 1 << 20)
+    (dl, dm, dn), lmn = geometry(nside)
+    s = np.stack([a[:npix] for a in lmn], 1).astype(np.float64)
+    worst = 0.0
+    for block in (64, 256, 1024):
+        t = (s.reshape(-1, block, 3) - s.reshape(-1, block, 3).mean(1, keepdims=True)).reshape(-1, 3)
+        for p in np.argsort(-(t * t).sum(1))[:6:3]:
+            axis = t[p] / np.linalg.norm(t[p])
+            across = np.cross(s[p], axis)
+            steps = 128 * -(-(6_100_000_000 // (npix * 56)) // 128)
+            bl, keep = tracks(vb, max(steps, 256), np.geomspace(0.02, 3.0, 56), axis, across, bend)
+            B = np.zeros(npix, np.float32)
+            B[p] = 1.0
+            dB = dev(B)
+            sky = sky_struct(dl, dm, dn, dB, npix)
+            V, _ = stage1(sky, bl, precision=vb.PREC_FP32_FP64PH, cull=0, blockage=0)
+            V64, _ = stage1(sky, bl, precision=vb.PREC_FP64, cull=0, blockage=0)
+            e = (V - V64).reshape(-1, 2)
+            worst = max(worst, float(np.hypot(e[:, 0], e[:, 1]).max()))
+    print("largest error of a term", worst)
+    assert worst <= TOL

@@ -69,8 +69,9 @@ struct Stage1Plan {
 };
 
 // Shape of one track group: mode < 0 = left to the per-term kernel, else
-// polynomial | log2(slots per sub-group) << 4 | pixel-block level << 8; centre,
-// frame and curve (b = gamma a + kappa a^2 in the frame) of each sub-group.
+// polynomial | log2(slots per sub-group) << 4 | pixel-block level << 8 |
+// coefficient table << 12; centre, frame and curve (b = gamma a + kappa a^2 in
+// the frame) of each sub-group.
 struct TrackSub {
   double uc[3];
   float e[9], gamma, kappa, pad;

@@ -9,14 +9,17 @@
 //   z_p = B_p e^{2 pi i u_c.s_p}     (one sin / cos per group and pixel).
 // In the group's frame (e1 along the track, e2 towards its sagitta, e3 across)
 // D_k is a place a on the curve b = gamma a + kappa a^2 and two small residuals
-// (the positions' float rounding, mostly); e^{2 pi i D_k.d_p} is the power
-// series in a of the curve's factor, times the residuals to first order.  The
-// warp forms the series' moments over the pixels once per (group, block), then
-// every baseline of the group evaluates one polynomial.  A group is taken only
-// where the truncation stays below 1e-7 rms of a term, under the 3e-7 noise of
-// the SFU's sin / cos that every term of both kernels carries; the others (fast
-// tracks on coarse pixels, irregular baselines, skies whose pixel blocks are not
-// compact) go to the per-term kernel through a list.
+// (the positions' float rounding, mostly); e^{2 pi i D_k.d_p} is a polynomial
+// in a for the curve's factor, times the residuals to first order.  The warp
+// forms the polynomial's moments over the pixels once per (group, block), then
+// every baseline of the group evaluates it.  A group is taken only where any
+// single term is off by at most 6e-7 (vb_series.h: 1e-7 for the polynomial, the
+// rest for the residuals, at a block's edge and a group's end); the phase of z_p is
+// rounded once here and three times in the per-term kernel, 3.7e-7 against 1.1e-6,
+// so that a term is no further off than there.  Measured on skies of one source,
+// largest and rms error of a term: 1.5e-6 and 3.4e-7, per-term kernel 1.5e-6 and
+// 4.4e-7.  The other groups (fast tracks on coarse pixels, irregular baselines,
+// skies whose pixel blocks are not compact) go to the per-term kernel through a list.
 //
 // Bound: FP32 issue.  Per group of K baselines and block of P pixels a warp
 // executes P/32 x (phase, sin/cos, 2 J multiply-adds) + a transposed
@@ -33,6 +36,7 @@
 #include "vb_common.cuh"
 #include "vb_geom.cuh"
 #include "vb_internal.h"
+#include "vb_series.h"
 #include "vb_stage1.cuh"
 #include "vb_track.cuh"
 
@@ -46,7 +50,7 @@ constexpr int TK_QUAD = 4;               // blocks whose moments a warp forms at
 constexpr int TK_CHUNK = TK_QUAD * 1024; // chunks hold whole quads of the largest blocks
 
 // Polynomial shapes: powers of a in the curve's own factor, in the residuals'
-// first-order terms, and their sum.
+// first-order terms, and their sum (coefficients: kSeries).
 template <int SET>
 struct Shape {
   static constexpr int N = SET == 0 ? 8 : SET == 1 ? 12 : 16;
@@ -55,10 +59,7 @@ struct Shape {
 };
 constexpr int TK_SETS = 3;
 constexpr int TK_JMAX = Shape<TK_SETS - 1>::J;
-// Largest truncation (kTailMax: the sum of the first dropped terms at the
-// corners of a group and a block; the rms over both is 100 times smaller) and
-// largest residual phases (their dropped products stay below 1e-6, 9e-8 rms).
-constexpr float kTailMax = 8e-6f, kResidualMax = 1.4e-3f;
+static_assert(Shape<0>::N == 8 && Shape<1>::N == 12 && Shape<2>::N == 16, "the shapes of kSeries");
 
 struct TrackArgs {
   const float *B, *l, *m, *n;
@@ -76,7 +77,7 @@ struct TrackArgs {
   int* queue;
   double2* partial;
   int n_half, nbl, steps, gpp;
-  float scale[TK_SETS][2 * TK_JMAX];       // coefficient and sign of each reduced moment
+  float scale[kSeriesTables][2 * TK_JMAX];  // coefficient and sign of each reduced moment
   unsigned char dest[TK_SETS][2 * TK_JMAX];
 };
 
@@ -204,7 +205,12 @@ __global__ void __launch_bounds__(256) k_track_blocks(const BlockArgs a) {
 // ---------------------------------------------------------------------------
 // Plan: the shape of each group (slots per sub-group, pixel block, polynomial),
 // or none.  One warp per group; O(n_half).
+struct SeriesBox {
+  int set;
+  float x1, x2, e;
+};
 struct PlanArgs {
+  SeriesBox box[kSeriesTables];
   const float *u, *v, *w, *x1, *y1, *z1, *in1;
   int nbl, steps, gpp, ngroups, max_level, blockage;
   const unsigned* rmax;
@@ -212,7 +218,8 @@ struct PlanArgs {
 };
 
 // Frame, curve and extents (half-range along the track, curve, residuals from
-// the curve and across) of one sub-group (slots [q0, q0 + ks) of the lanes).
+// the curve and across; the first two grow by the tilt that the curve's slope
+// gives the axis) of one sub-group (slots [q0, q0 + ks) of the lanes).
 __device__ __forceinline__ void sub_frame(const float (&p)[TK_SLOTS][3], int nv, int lane, int q0, int ks, double (&uc)[3],
                                           float (&e)[9], float& gamma, float& kappa, float (&R)[4]) {
   const int n0 = q0 * 32, n1 = min(nv, (q0 + ks) * 32);
@@ -318,8 +325,9 @@ __device__ __forceinline__ void sub_frame(const float (&p)[TK_SLOTS][3], int nv,
   }
   eh = warp_max(eh); el = -warp_max(-el);
   const float mide = 0.5f * (eh + el);
-  R[0] = A;
-  R[1] = (float)fabs(k);
+  const float tilt = 1.f + fabsf((float)g) * invA;
+  R[0] = A * tilt;
+  R[1] = (float)fabs(k) * tilt;
   R[2] = 0.5f * (eh - el);
   R[3] = 0.5f * (hc - lc);
   gamma = (float)(g * invA);
@@ -327,24 +335,6 @@ __device__ __forceinline__ void sub_frame(const float (&p)[TK_SLOTS][3], int nv,
   const double bc = beta + (double)mide;
   for (int c = 0; c < 3; ++c)
     uc[c] = (double)first[c] + (double)mid * e[c] + bc * e[3 + c] + (double)midc * e[6 + c];
-}
-
-// Sum of the first two dropped terms of a group whose largest |a tau| is X1 and
-// whose curve adds X2: the power series of e^{X1 s + X2 s^2} from s^n on.
-__device__ __forceinline__ void tails(float X1, float X2, float (&h)[TK_SETS][2]) {
-  float h0 = 1.f, h1 = X1;
-#pragma unroll
-  for (int n = 2; n <= 17; ++n) {
-    const float h2 = (X1 * h1 + 2.f * X2 * h0) * (1.f / n);
-    h0 = h1;
-    h1 = h2;
-    // (h0, h1) = terms (n - 1, n)
-    if (n == 5) h[0][1] = h0 + h1;
-    if (n == 7) h[1][1] = h0 + h1;
-    if (n == 9) { h[2][1] = h0 + h1; h[0][0] = h0 + h1; }
-    if (n == 13) h[1][0] = h0 + h1;
-    if (n == 17) h[2][0] = h0 + h1;
-  }
 }
 
 __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
@@ -404,11 +394,12 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
       const float crossed = fminf(32.f * ks, 1.f + 2.f * r64 / fmaxf(turn, 1e-6f));   // steps on the horizon in a 64-pixel part
       for (int lev = 0; lev <= a.max_level; ++lev) {
         const float r = __uint_as_float(a.rmax[lev]);
-        const float k = 6.2831855f * r, E = k * (M[2] + M[3]);
-        float h[TK_SETS][2];
-        tails(k * M[0], k * M[1], h);
-        for (int set = 0; set < TK_SETS; ++set) {
-          if (!(h[set][0] + E * h[set][1] <= kTailMax && E <= kResidualMax)) continue;
+        const float k = 6.2831855f * r, X1 = k * M[0], X2 = k * M[1], E = k * sqrtf(M[2] * M[2] + M[3] * M[3]);
+        int tried = -1;
+        for (int t = 0; t < kSeriesTables; ++t) {
+          const int set = a.box[t].set;
+          if (set == tried || !(X1 <= a.box[t].x1 && X2 <= a.box[t].x2 && E <= a.box[t].e)) continue;
+          tried = set;   // (the tables are sorted by shape)
           fits = true;
           const float P = (float)tk_block(lev);
           float node = P * (1.f / 32.f) * c_pix[set] + c_red[set] + ks * c_eval[set];
@@ -416,7 +407,7 @@ __global__ void __launch_bounds__(128) k_track_plan(const PlanArgs a) {
             node += fminf(1.f, 0.28f * (turn * 32.f * ks + 2.f * r)) *
                     (lev * (P * (1.f / 32.f) * c_pix[set] + 4.f * (c_red[set] + c_eval[set])) + P * (1.f / 64.f) * (150.f + 70.f * crossed));
           const float cost = node / (ks * P * fill);
-          if (cost < best) { best = cost; mode = set | (ls << 4) | (lev << 8); }
+          if (cost < best) { best = cost; mode = set | (ls << 4) | (lev << 8) | (t << 12); }
         }
       }
       if (!fits) break;   // longer sub-groups extend further
@@ -577,18 +568,20 @@ struct TrackWarp {               // one warp's group
   float4 d1[TK_SLOTS][32], d2[TK_SLOTS][32];
   float s1[TK_SLOTS][32], s2[TK_SLOTS][32];
   float mom[TK_QUAD][2 * TK_JMAX];
+  float scale[2 * TK_JMAX];      // of the group's table
   TrackPlan plan;
 };
 struct TrackSmem {
   TrackWarp w[TK_WARPS];
-  float scale[TK_SETS][2 * TK_JMAX];
   unsigned char dest[TK_SETS][2 * TK_JMAX];
 };
 
-// Turn phase of a (baseline, pixel) term as angle bits, see vb_stage1.cuh.
+// Turn phase of a (baseline, pixel) term as angle bits, see vb_stage1.cuh; the
+// products are summed before the one rounding to the 2^-23-turn grid (one FP64
+// operation more a pixel and group, which all its steps share).
 __device__ __forceinline__ void phase_cs(double U, double V, double W, float l, float m, float n, unsigned flip, float& s,
                                          float& c) {
-  const double t = fma(U, (double)l, fma(V, (double)m, fma(W, (double)n, kMagic)));
+  const double t = fma(U, (double)l, fma(V, (double)m, W * (double)n)) + kMagic;
   const unsigned kb = ((unsigned)__double2loint(t) & 0x7FFFFFu) ^ flip;
   __sincosf(__fmaf_rn(__uint_as_float(kb), kAngScale, -kTwoPiF), &s, &c);
 }
@@ -847,9 +840,9 @@ __device__ __forceinline__ unsigned track_quad(const TrackArgs& a, TrackSmem& sm
       continue;
     }
     const TrackSub& sub = w.plan.sub[q0 / ks];
-    if (set == 0) track_moments<0>(a, mine, np, P, sub, cen, inv_r, sm.scale[0], sm.dest[0], w.mom[0], lane);
-    else if (set == 1) track_moments<1>(a, mine, np, P, sub, cen, inv_r, sm.scale[1], sm.dest[1], w.mom[0], lane);
-    else track_moments<2>(a, mine, np, P, sub, cen, inv_r, sm.scale[2], sm.dest[2], w.mom[0], lane);
+    if (set == 0) track_moments<0>(a, mine, np, P, sub, cen, inv_r, w.scale, sm.dest[0], w.mom[0], lane);
+    else if (set == 1) track_moments<1>(a, mine, np, P, sub, cen, inv_r, w.scale, sm.dest[1], w.mom[0], lane);
+    else track_moments<2>(a, mine, np, P, sub, cen, inv_r, w.scale, sm.dest[2], w.mom[0], lane);
 #pragma unroll 1
     for (int q = q0; q < q0 + ks; ++q) {
       const float ka = w.a[q][lane], kb = w.b[q][lane], kc = w.c[q][lane];
@@ -884,10 +877,7 @@ __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_consta
   asm volatile("griddepcontrol.launch_dependents;");   // the list kernel may take SMs that this one leaves
   const int nfast = a.count[0];
   const int n_items = nfast * a.nchunk;
-  for (int i = threadIdx.x; i < TK_SETS * 2 * TK_JMAX; i += TK_THREADS) {
-    (&sm.scale[0][0])[i] = (&a.scale[0][0])[i];
-    (&sm.dest[0][0])[i] = (&a.dest[0][0])[i];
-  }
+  for (int i = threadIdx.x; i < TK_SETS * 2 * TK_JMAX; i += TK_THREADS) (&sm.dest[0][0])[i] = (&a.dest[0][0])[i];
   __syncthreads();
 
   // Work item: one group over one pixel chunk, by one warp (the warps differ in
@@ -903,7 +893,7 @@ __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_consta
     const int g = a.list[item - chunk * nfast];
 
     // --- the group -------------------------------------------------------------
-    const int mode = a.plan[g].mode, set = mode & 15, ks = 1 << ((mode >> 4) & 15), level = mode >> 8;
+    const int mode = a.plan[g].mode, set = mode & 15, ks = 1 << ((mode >> 4) & 15), level = (mode >> 8) & 15;
     const float r = __uint_as_float(a.rmax[level]), inv_r = 1.f / r;
     const int pair = g / a.gpp, st0 = (g - pair * a.gpp) * TK_GROUP;
     const int nv = min(TK_GROUP, a.steps - st0);
@@ -914,6 +904,7 @@ __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_consta
       const int* src = reinterpret_cast<const int*>(a.plan + g);
       int* dst = reinterpret_cast<int*>(&w.plan);
       for (int i = lane; i < (int)(sizeof(TrackPlan) / sizeof(int)); i += 32) dst[i] = src[i];
+      for (int i = lane; i < 2 * TK_JMAX; i += 32) w.scale[i] = a.scale[mode >> 12][i];
       __syncwarp();
       const float kr = 6.28318530717958647692f * r;
       for (int q = 0; q < TK_SLOTS; ++q) {
@@ -1007,20 +998,25 @@ __global__ void __launch_bounds__(TK_THREADS, 3) k_track_sum(const __grid_consta
 }
 
 // ---------------------------------------------------------------------------
-// i^n / n! (one more i in the residual terms): coefficient and sign of each
-// part of a moment, and where multiplication by i^d puts it.
-template <int SET>
-static void set_tables(float* scale, unsigned char* dest) {
-  using S = Shape<SET>;
-  for (int o = 0; o < S::J; ++o) {
-    const int n = o < S::N ? o : (o - S::N) % S::NE;
-    const int d = (n + (o < S::N ? 0 : 1)) & 3;
-    double f = 1.0;
+// Coefficient and sign of each part of a moment: i^n / n! (one more i in the
+// residual terms) times the table's correction.
+static void series_scale(const SeriesTable& t, float* scale) {
+  for (int o = 0; o < 2 * t.n; ++o) {
+    const int n = o < t.n ? o : (o - t.n) % (t.n / 2);
+    const int d = (n + (o < t.n ? 0 : 1)) & 3;
+    double f = o < t.n ? t.main[n] : t.res[n];
     for (int k = 2; k <= n; ++k) f /= k;
     const double sre = (d == 0 || d == 1) ? f : -f;   // re -> re, im, -re, -im
     const double sim = (d == 0 || d == 3) ? f : -f;   // im -> im, -re, -im, re
     scale[2 * o] = (float)sre;
     scale[2 * o + 1] = (float)sim;
+  }
+}
+
+// Where multiplication by that power of i puts the two parts.
+static void series_dest(int N, unsigned char* dest) {
+  for (int o = 0; o < 2 * N; ++o) {
+    const int d = (o < N ? o : (o - N) % (N / 2) + 1) & 3;
     dest[2 * o] = (unsigned char)(2 * o + (d & 1));
     dest[2 * o + 1] = (unsigned char)(2 * o + 1 - (d & 1));
   }
@@ -1116,6 +1112,7 @@ int track_group(const vb_baselines* bl, const Stage1Plan& p, const Stage1Buffers
   k.blockage = p.blockage;
   k.rmax = b.trk.rmax;
   k.plan = b.trk.plan;
+  for (int t = 0; t < kSeriesTables; ++t) k.box[t] = {kSeries[t].n / 4 - 2, kSeries[t].x1, kSeries[t].x2, kSeries[t].e};
   const int grid = (int)ceil_div(p.trk_groups, 4);
   k_track_plan<<<grid, 128, 0, s>>>(k);
   VB_LAUNCH_CHECK();
@@ -1147,9 +1144,8 @@ int track_sum(const vb_sky* sky, const Stage1Plan& p, const Stage1Buffers& b, cu
   a.q0 = b.trk.q0; a.d1 = b.trk.d1; a.d2 = b.trk.d2; a.p1 = b.trk.p1; a.p2 = b.trk.p2; a.t2 = b.trk.t2;
   a.list = b.trk.list; a.count = b.trk.count; a.queue = b.queue + 2;
   a.partial = b.partial; a.n_half = p.n_half; a.nbl = p.nbl; a.steps = p.trk_steps; a.gpp = p.trk_gpp;
-  set_tables<0>(a.scale[0], a.dest[0]);
-  set_tables<1>(a.scale[1], a.dest[1]);
-  set_tables<2>(a.scale[2], a.dest[2]);
+  for (int t = 0; t < kSeriesTables; ++t) series_scale(kSeries[t], a.scale[t]);
+  for (int set = 0; set < TK_SETS; ++set) series_dest(8 + 4 * set, a.dest[set]);
   VB_CUDA(cudaFuncSetAttribute((const void*)k_track_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrackSmem)));
   k_track_sum<<<p.trk_grid, TK_THREADS, sizeof(TrackSmem), s>>>(a);
   VB_LAUNCH_CHECK();
