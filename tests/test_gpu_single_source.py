@@ -1,21 +1,22 @@
-"""Factored sums with one term that matters: a sky of one source (stage 1).  Errors then
-cannot cancel, so this is the largest error of a term.
+"""Factored sums with one term that matters: a sky of one source (stage 1), one visibility
+(stage 2).  Errors then cannot cancel, so this is the largest error of a term.
 
-The pairs move along tracks of one direction at 56 speeds, so that every polynomial is met
-at the ends of its range, and the source is the pixel that lies farthest along the tracks
-from its block's centre.
+The pairs move along tracks of one direction at many speeds, so that every polynomial is
+met at the ends of its range.  Stage 1: the source is the pixel that lies farthest along the
+tracks from its block's centre; stage 2: the visibility is the last of a cluster.
 
 Tolerance for |exp(i phi)|: half a step of the 2^-23-turn phase grid 3.7e-7, the angle in
 float32 2.4e-7 and its fl(2 pi) 1.7e-7, the SFU's sine and cosine 6e-7, polynomials
 6e-7 and their float sums 5e-7 (powers up to 2.5^n / n!), 2.5e-6 in all; the
-per-term kernel's own bound, with three roundings of the phase, is 2.1e-6.
+per-term kernel's own bound, with three roundings of the phase, is 2.1e-6.  Stage 2:
+polynomials 1.5e-7 and their float sums 2e-7, 1.8e-6 in all.
 """
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
-from gpu_util import dev, geometry, sky_struct, stage1
+from gpu_util import dev, geometry, sky_struct, stage1, stage2, zeros
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +62,30 @@ def test_one_source(vb, gpu, nside, bend):
             worst = max(worst, float(np.hypot(e[:, 0], e[:, 1]).max()))
     print("largest error of a term", worst)
     assert worst <= TOL
+
+
+def test_one_visibility(vb, gpu):
+    npix, steps, pairs = 2200000, 500, 28
+    (dl, dm, dn), _ = geometry(512)
+    sky = sky_struct(dl, dm, dn, dl, npix)
+    axis, across = np.array([0.8, 0.6, 0.0]), np.array([-0.6, 0.8, 0.0])
+    # cells of 0.1 wavelengths: each step of a track has its own, clusters of 32 steps
+    bl, keep = tracks(vb, steps, np.geomspace(0.15, 0.7, pairs), axis, across, 0.02)
+    ends = [zeros(bl.n_full) for _ in range(8)]
+    for k, b in zip(("x1", "y1", "z1", "invn1", "x2", "y2", "z2", "invn2"), ends):
+        setattr(bl, k, b.ptr)
+    kw = dict(mirror=1, blockage=0, lam=1.0, bl_max=819.2, grid_res=16385)
+    worst, seen = 0.0, 0
+    for pair in range(pairs):
+        V = np.zeros((steps * pairs, 2), np.float32)
+        V[(160 + 31 * (pair % 2)) * pairs + pair] = (0.8, -0.6)
+        dV = dev(V)
+        C1, _, p1, _ = stage2(sky, bl, dV, [0], [steps], precision=vb.PREC_FP32_FP64PH, **kw)
+        C64, _, p64, _ = stage2(sky, bl, dV, [0], [steps], precision=vb.PREC_FP64, **kw)
+        assert p1 == p64
+        if not C64.any():
+            continue          # (off the grid)
+        seen += 1
+        worst = max(worst, float(np.abs(C1.astype(np.float64) - C64).max()) * p64[0]["nuniq"])
+    print("largest error of a term", worst)
+    assert seen > pairs // 2 and worst <= 1.8e-6

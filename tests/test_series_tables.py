@@ -52,3 +52,29 @@ def test_any_single_term_is_within_the_bound(k):
     y = np.sqrt(1 - c * c) * e            # the residual phase leaves to the block's edge what the track does not take
     t = np.abs(series(res, X1 * c, X2 * s) - f) * y
     assert (t + y * y / 2).max() <= 5e-7
+
+
+def cluster_tables():
+    text = (ROOT / "viss_optimize_ws_b200" / "csrc" / "vb_series.h").read_text()
+    body = text[text.index("kClusters[] = {"):]
+    return [(int(m[1]), float(np.float32(m[2])), float(np.float32(m[3])), np.array(m[4].split(","), float))
+            for m in re.finditer(r"\{(\d+), (%s)f, (%s)f,\s*\{([^}]*)\}\}" % (NUM, NUM), body)]
+
+
+CLUSTERS = cluster_tables()
+
+
+BOUNDS = (3e-8, 3e-8, 6e-8, 6e-8, 1.5e-7, 1.5e-7)
+
+
+@pytest.mark.parametrize("k", range(len(CLUSTERS)))
+def test_any_single_term_of_a_cluster_is_within_the_bound(k):
+    assert len(CLUSTERS) == len(BOUNDS)
+    shape, X1, X2, coef = CLUSTERS[k]
+    rows = ((10, 9, 7, 5, 1), (9, 8, 7, 5, 3))[shape]
+    assert coef.size == sum(rows) == 32
+    r, th = np.meshgrid(np.linspace(0, 1, 61), np.linspace(0, 2 * math.pi, 361))
+    x, y = X1 * r * np.cos(th), X2 * r * np.sin(th)
+    it = iter(coef)
+    s = sum(next(it) * (1j * x) ** i / math.factorial(i) * (1j * y) ** c / math.factorial(c) for c, n in enumerate(rows) for i in range(n))
+    assert np.abs(s - np.exp(1j * (x + y))).max() <= BOUNDS[k]

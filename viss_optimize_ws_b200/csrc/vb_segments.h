@@ -3,11 +3,7 @@
 #pragma once
 #include <cstdint>
 
-#ifdef __CUDACC__
-#define VB_HOST_DEVICE __host__ __device__
-#else
-#define VB_HOST_DEVICE
-#endif
+#include "vb_host_device.h"
 
 namespace vb {
 

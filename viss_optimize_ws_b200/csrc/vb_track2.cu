@@ -9,10 +9,13 @@
 //   P = sum_g V_g e^{2 pi i D_g.s_c} e^{i (x_g tau + y_g eta)},
 // where (x, y) is the cell's place in the cluster's frame and (tau, eta) the
 // pixel's in the block.  e^{i (x tau + y eta)} is a polynomial of 32 terms
-// (Chebyshev-economised on the cluster's intervals, 1e-7 rms): a warp forms its
-// coefficients once per (cluster, block), a lane per group, and every pixel
-// evaluates it.  Clusters that no polynomial fits and groups outside clusters
-// stay on k_recon_rec.
+// (vb_series.h, any single term within 1.5e-7): a warp forms its coefficients once
+// per (cluster, block), a lane per group, and every pixel evaluates it.  The
+// phase of a pixel's factor is rounded once to the 2^-23-turn grid, where
+// k_recon_rec rounds twice, 3.7e-7 against 7.5e-7, so that a term is no further off
+// than there (1.5 % of the kernel's time).  Measured with one visibility, largest and
+// rms error of a term: 1.1e-6 and 2.4e-7, k_recon_rec 1.2e-6 and 2.7e-7.  Clusters
+// that no polynomial fits and groups outside clusters stay on k_recon_rec.
 //
 // Bound: FP32 issue (per cluster and 1024 pixels: 4 x (32 groups' classes, FP64
 // rotation, 64 products, transposed reduction) and 32 x (phase, sin/cos, 64
@@ -28,6 +31,7 @@
 #include "vb_geom.cuh"
 #include "vb_internal.h"
 #include "vb_segments.h"
+#include "vb_series.h"
 #include "vb_stage1.cuh"
 #include "vb_stage2.cuh"
 #include "vb_track.cuh"
@@ -41,28 +45,24 @@ constexpr int G2_LEVEL = 1;             // TrackNode level of 256 pixels
 constexpr int G2_TRACKS = 4096;         // largest pairs (signed pairs) per step
 constexpr int G2_MIN = 10;              // groups from which a cluster pays (about 380 / 8 + 70 cycles for each 32 pixels)
 
-// Polynomial shapes: powers of tau for eta^0.. eta^4, the intervals of |x tau|
-// and |y eta| they are economised on, and the clusters they take.  X1, X2 are the
-// largest |x tau| and |y eta| at the sky's largest block; a typical block is 3/4
-// of that, so that clusters somewhat past the economised intervals still stay at
-// 5e-8 rms over the sky (1e-7 allowed; measured in double over both ranges).
-template <int SET>
+// Polynomial shapes: powers of tau for eta^0.. eta^4.
+template <int SHAPE>
 struct Poly {
-  static constexpr int J = 32, NC = 5;
-  __host__ __device__ static constexpr int N(int c) {
-    return SET == 0 ? (c == 0 ? 10 : c == 1 ? 9 : c == 2 ? 7 : c == 3 ? 5 : 1) : (c == 0 ? 9 : c == 1 ? 8 : c == 2 ? 7 : c == 3 ? 5 : 3);
-  }
+  static constexpr int NC = 5;
+  __host__ __device__ static constexpr int N(int c) { return cluster_row(SHAPE, c); }
 };
-constexpr int G2_SETS = 2, G2_J = 32;
-__host__ __device__ constexpr float g2_box(int set, int axis) {
-  return set == 0 ? (axis == 0 ? 1.4f : 0.11f) : (axis == 0 ? 1.2f : 0.09f);
+constexpr int G2_SHAPES = 2, G2_J = kClusterTerms;
+// Shape of each table, a bit each.
+constexpr unsigned shape_bits() {
+  unsigned m = 0;
+  for (int t = 0; t < kClusterTables; ++t) m |= (unsigned)kClusters[t].shape << t;
+  return m;
 }
-__device__ __forceinline__ bool g2_takes(int set, float X1, float X2) {
-  return set == 0 ? X1 <= 1.9f && X2 <= 0.075f : X1 <= 1.5f && X2 <= 0.16f && X2 <= 0.16f - 0.24f * (X1 - 1.25f);
-}
+constexpr unsigned G2_SHAPE_BITS = shape_bits();
 
 // --- clusters -------------------------------------------------------------------
 struct ClusterArgs {
+  float2 box[kClusterTables];   // largest |x tau|, |y eta| of each table
   const unsigned long long* skeys;
   const int *svals, *start, *ngroups;
   const vb_seg_params* sp;
@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(128) k_cluster_plan(const ClusterArgs a) {
     q.seg = whole.seg;
     q.set = -1;
     if (!own || l1 - l0 < G2_MIN / 2) return false;
-    for (int s = G2_SETS - 1; s >= 0; --s)
-      if (g2_takes(s, X1, X2)) q.set = s;
+    for (int t = kClusterTables - 1; t >= 0; --t)
+      if (X1 <= a.box[t].x && X2 <= a.box[t].y) q.set = t;
     if (q.set < 0) return false;
     const double mx = 0.5 * ((double)xh + xl), my = 0.5 * ((double)yh + yl);
     q.uc[0] = f0[0] + mx * e1[0] + my * e2[0];
@@ -332,16 +332,16 @@ struct TrackReconArgs {
   int* queue;
   double* Cpart;       // [rows][npix]
   unsigned* Wpart;
-  float scale[G2_SETS][2 * G2_J];
-  unsigned char dest[G2_SETS][2 * G2_J];
+  float scale[kClusterTables][2 * G2_J];
+  unsigned char dest[G2_SHAPES][2 * G2_J];
 };
 
 // Coefficients of one (cluster, block): lane = group, value w = V e^{2 pi i D.s_c}
 // (zero for the lanes that do not take part).
-template <int SET>
+template <int SHAPE>
 __device__ __forceinline__ void cluster_moments(float wr, float wi, float x, float y, const float* scale, const unsigned char* dest,
                                                 float* mom, int lane) {
-  using P = Poly<SET>;
+  using P = Poly<SHAPE>;
   float v[2 * G2_J];
   int o = 0;
 #pragma unroll
@@ -370,10 +370,10 @@ __device__ __forceinline__ void cluster_moments(float wr, float wi, float x, flo
 
 // The polynomial at a thread's four pixels (of one block: each coefficient is
 // loaded once for the four, whose chains are independent).
-template <int SET>
+template <int SHAPE>
 __device__ __forceinline__ void cluster_eval(const float* mom, const float (&tau)[G2_PPT], const float (&eta)[G2_PPT],
                                              float2 (&out)[G2_PPT]) {
-  using P = Poly<SET>;
+  using P = Poly<SHAPE>;
   const f2* m = reinterpret_cast<const f2*>(mom);
   f2 t2[G2_PPT], r[G2_PPT];
 #pragma unroll
@@ -412,17 +412,15 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
   __shared__ ClusterStage s_cl[G2_STAGE];
   __shared__ __align__(16) int s_clu[2][G2_STAGE][kClusterWords];   // this step's clusters and the next's
   __shared__ TrackNode s_node[G2_PPT];
-  __shared__ float s_scale[G2_SETS][2 * G2_J];
-  __shared__ unsigned char s_dest[G2_SETS][2 * G2_J];
+  __shared__ float s_scale[kClusterTables][2 * G2_J];
+  __shared__ unsigned char s_dest[G2_SHAPES][2 * G2_J];
   __shared__ int s_item;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   asm volatile("griddepcontrol.launch_dependents;");   // k_recon_rec may take SMs that this one leaves
   const int nc = a.count[0], nd = a.count[1];
   if (nc == 0) return;
-  for (int i = threadIdx.x; i < G2_SETS * 2 * G2_J; i += G2_THREADS) {
-    (&s_scale[0][0])[i] = (&a.scale[0][0])[i];
-    (&s_dest[0][0])[i] = (&a.dest[0][0])[i];
-  }
+  for (int i = threadIdx.x; i < kClusterTables * 2 * G2_J; i += G2_THREADS) (&s_scale[0][0])[i] = (&a.scale[0][0])[i];
+  for (int i = threadIdx.x; i < G2_SHAPES * 2 * G2_J; i += G2_THREADS) (&s_dest[0][0])[i] = (&a.dest[0][0])[i];
   const float r = __uint_as_float(a.rmax[G2_LEVEL]), inv_r = 1.f / r, kr = 6.28318530717958647692f * r;
   const int per_row = (nc + a.rows - 1) / a.rows;
   const int n_items = a.rows * a.nblocks;
@@ -523,8 +521,8 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
             wi = (float)fma((double)vx, es, (double)vy * ec);
           }
           const float xx = c == kClsVis ? x : 0.f, yy = c == kClsVis ? y : 0.f;
-          if (set == 0) cluster_moments<0>(wr, wi, xx, yy, s_scale[0], s_dest[0], s_mom[warp][q], lane);
-          else cluster_moments<1>(wr, wi, xx, yy, s_scale[1], s_dest[1], s_mom[warp][q], lane);
+          if (!(G2_SHAPE_BITS >> set & 1)) cluster_moments<0>(wr, wi, xx, yy, s_scale[set], s_dest[0], s_mom[warp][q], lane);
+          else cluster_moments<1>(wr, wi, xx, yy, s_scale[set], s_dest[1], s_mom[warp][q], lane);
         }
       }
       if (lane < kClusterWords) s_clu[buf ^ 1][warp][lane] = word;
@@ -540,7 +538,7 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
           mp[q] = fma((double)fb, (double)nf[q], (double)mf[q]);
         }
         auto angle = [&](double A, double B, int q, bool odd, float& s, float& c) {
-          const double t = fma(A, lp[q], fma(B, mp[q], kMagic));
+          const double t = fma(A, lp[q], B * mp[q]) + kMagic;   // one rounding to the grid
           const unsigned kb = ((unsigned)__double2loint(t) & 0x7FFFFFu) ^ (odd ? 0x4B400000u : 0x4B000000u);
           __sincosf(__fmaf_rn(__uint_as_float(kb), kAngScale, -kTwoPiF), &s, &c);
         };
@@ -557,7 +555,7 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
               tau[q] = fmaf(dx, st.e1[0], fmaf(dy, st.e1[1], dz * st.e1[2]));
               eta[q] = fmaf(dx, st.e2[0], fmaf(dy, st.e2[1], dz * st.e2[2]));
             }
-            if (st.set == 0) cluster_eval<0>(s_mom[k][wq], tau, eta, h);
+            if (!(G2_SHAPE_BITS >> st.set & 1)) cluster_eval<0>(s_mom[k][wq], tau, eta, h);
             else cluster_eval<1>(s_mom[k][wq], tau, eta, h);
 #pragma unroll
             for (int q = 0; q < G2_PPT; ++q) {
@@ -608,49 +606,30 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
   }
 }
 
-// Coefficients g_n (n < count) of the polynomial sum g_n (i y)^n of degree
-// count - 1 nearest to e^{iy} on |y| <= X: the truncated Chebyshev series,
-// expanded in powers.
-static void economised(double X, int count, double* g) {
-  constexpr int M = 64;
-  const double pi = 3.14159265358979323846;
-  double c[32] = {};
-  for (int n = 0; n < count; ++n) {
-    double sum = 0.0;   // even orders: the series of cos, odd: of sin
-    for (int k = 0; k < M; ++k) {
-      const double th = pi * (k + 0.5) / M, y = X * std::cos(th);
-      sum += ((n & 1) ? std::sin(y) : std::cos(y)) * std::cos(n * th);
-    }
-    c[n] = (n ? 2.0 : 1.0) / M * sum;
-  }
-  double t0[34] = {1.0}, t1[34] = {0.0, 1.0}, p[34] = {};   // T_n, T_{n+1} in powers of y / X
-  for (int n = 0; n < count; ++n) {
-    for (int i = 0; i <= n; ++i) p[i] += c[n] * t0[i];
-    double t2[34] = {};
-    for (int i = 0; i < 33; ++i) t2[i + 1] = 2.0 * t1[i];
-    for (int i = 0; i < 34; ++i) { t2[i] -= t0[i]; t0[i] = t1[i]; t1[i] = t2[i]; }
-  }
-  double xn = 1.0;
-  for (int n = 0; n < count; ++n, xn *= X) g[n] = (((n / 2) & 1) ? -p[n] : p[n]) / xn;
-}
-
-template <int SET>
-static void poly_tables(float* scale, unsigned char* dest) {
-  using P = Poly<SET>;
-  double col[8], pow[32];
-  economised(g2_box(SET, 1), P::NC, col);
-  int o = 0;
-  for (int c = 0; c < P::NC; ++c) {
-    economised(g2_box(SET, 0), P::N(c), pow);
-    for (int i = 0; i < P::N(c); ++i, ++o) {
-      const double f = col[c] * pow[i];
-      const int d = (i + c) & 3;   // i^(i + c) times (re, im)
+// Coefficient and sign of each part of a moment, i^(k + c) / (k! c!) times the
+// table's correction, and where multiplication by that power of i puts it.
+static void poly_scale(const ClusterTable& t, float* scale) {
+  double col = 1.0;
+  for (int c = 0, o = 0; c < 5; ++c) {
+    if (c) col /= c;
+    double row = 1.0;
+    for (int k = 0; k < cluster_row(t.shape, c); ++k, ++o) {
+      if (k) row /= k;
+      const double f = t.coef[o] * col * row;
+      const int d = (k + c) & 3;
       scale[2 * o] = (float)((d == 0 || d == 1) ? f : -f);
       scale[2 * o + 1] = (float)((d == 0 || d == 3) ? f : -f);
-      dest[2 * o] = (unsigned char)(2 * o + (d & 1));
-      dest[2 * o + 1] = (unsigned char)(2 * o + 1 - (d & 1));
     }
   }
+}
+
+static void poly_dest(int shape, unsigned char* dest) {
+  for (int c = 0, o = 0; c < 5; ++c)
+    for (int k = 0; k < cluster_row(shape, c); ++k, ++o) {
+      const int d = (k + c) & 1;
+      dest[2 * o] = (unsigned char)(2 * o + d);
+      dest[2 * o + 1] = (unsigned char)(2 * o + 1 - d);
+    }
 }
 
 // Clusters are in use for the FP32 sum with FP64 phase over representatives or
@@ -700,6 +679,7 @@ int cluster_group(const Stage2Plan& p, const ClusterBuffers& x, const unsigned l
   a.n_keyed = p.n_keyed_total; a.ntrk = p.trk_ntrk; a.nseg = p.nseg; a.entries = p.trk_entries;
   a.rmax = x.rmax; a.steps = x.steps; a.slots = x.slots; a.order = x.order; a.dst = x.dst; a.list = x.list; a.count = x.count; a.table = x.table; a.clu = x.clu;
   a.spd = x.spd;
+  for (int t = 0; t < kClusterTables; ++t) a.box[t] = make_float2(kClusters[t].x1, kClusters[t].x2);
   VB_CUDA(cudaMemsetAsync(x.slots, 0xff, (size_t)p.n_keyed_total * sizeof(int), s));
   VB_CUDA(cudaMemsetAsync(x.table, 0, 2 * (size_t)p.trk_entries * sizeof(GroupCluster), s));
   const int g = (int)std::min<int64_t>(ceil_div(p.n_keyed_total, 256), (int64_t)sm_count() * 16);
@@ -726,8 +706,8 @@ int cluster_sum(const vb_sky* sky, const Stage2Plan& p, const ClusterBuffers& x,
   a.node = x.node[G2_LEVEL]; a.rmax = x.rmax; a.clu = x.clu; a.count = x.count; a.sp = sp; a.rec = rec;
   a.nrec = ngroups;
   a.queue = queue; a.Cpart = Cpart; a.Wpart = Wpart;
-  poly_tables<0>(a.scale[0], a.dest[0]);
-  poly_tables<1>(a.scale[1], a.dest[1]);
+  for (int t = 0; t < kClusterTables; ++t) poly_scale(kClusters[t], a.scale[t]);
+  for (int shape = 0; shape < G2_SHAPES; ++shape) poly_dest(shape, a.dest[shape]);
   const int grid = (int)std::min<int64_t>((int64_t)sm_count() * 2, (int64_t)p.trk_rows * p.trk_blocks);
   k_recon_track<<<grid, G2_THREADS, 0, s>>>(a);
   VB_LAUNCH_CHECK();
