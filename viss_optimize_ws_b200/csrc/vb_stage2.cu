@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(S2_THREADS, 2) k_recon_rec(const ReconArgs a) 
 // (gathered once per CTA, where every warp used to fetch each member's endpoints
 // itself), each member classified against the block's cone, so that hidden
 // members are skipped and visible ones take no test; a group without any member
-// left costs no sine.  1.48 -> 0.86 ms (49,152 pixels, four samples, signed set).
+// left costs no sine.  1.57 -> 0.54 ms (49,152 pixels, four samples, signed set).
 constexpr int M_GROUPS = 64, M_MEMBERS = S2_THREADS, M_PPT = 2;
 struct MemberRec {
   float4 p1, p2;          // (x, y, z, invn) of the endpoints
