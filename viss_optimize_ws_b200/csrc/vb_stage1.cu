@@ -829,8 +829,15 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
   q.npix = sky->npix;
   q.n_half = bl->n_full / 2;
   q.nbl = bl->nbl;
-  // below about 2e7 terms the cones cost as much as they save
-  q.no_cones = (double)q.n_half * (double)q.npix < 2e7;
+  // Cones of a small call cost what they save: from 2e7 terms.  With / without, us
+  // (one B200, 28 pairs): 49,152 pixels, 2.8e7 terms 66 / 71, 5.5e7 80 / 95, 1.1e8
+  // 108 / 138; 20,000 pixels, 2.2e7 57 / 54, 9.0e7 100 / 106; 12,288 pixels, 5.5e7
+  // 76 / 70, 1.1e8 112 / 134.  On a sky of up to four tiles a sub-tile mostly holds
+  // the horizon, and the line lies at more terms the fewer its pixels: 3,072 pixels,
+  // 5.5e7 87 / 69, 1.1e8 143 / 123, 2.2e8 236 / 229, 4.3e8 419 / 441.
+  const double terms = (double)q.n_half * (double)q.npix;
+  const bool coarse = q.npix < 4096;
+  q.no_cones = terms < 2e7 || (coarse && terms * (double)q.npix < 1.5e12);
 
   int stage = o->stage_pix > 0 ? o->stage_pix : 1024;
   if (!is_pow2(stage) || stage < 32 || stage > 2048)
@@ -891,7 +898,13 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
   // A small call has fewer (baseline tile, cull tile) items than the chip has
   // room for: items then take parts of a cull tile, halved until there are 4 for
   // each resident CTA (their work differs with the horizon), but below 256
-  // pixels only while a CTA has none, since each repeats the baselines' set-up.
+  // pixels only while a CTA has none, since each repeats the baselines' set-up;
+  // until there are 2 on such a coarse sky where a part tests every pixel, or
+  // repeats the FP64 cone test of its tile.  Whole tiles over parts until 4 / until
+  // 2, at 1.4, 2 and 2.8 whole tiles for each CTA: VB_CULL_EXACT, 3,072 pixels
+  // 0.92 / 0.96, 1.10 / 1.20, 0.98 / 1.01, but 49,152 pixels 1.00 / 1.03, 1.05 / 1.09,
+  // 1.05 / 1.03; VB_CULL_NONE, 3,072 pixels 0.93 / 0.98, 1.16 / 1.21, 0.98 / 1.00, but
+  // 5,000 pixels 1.10 / 1.02, 1.31 / 1.34, 1.22 / 1.19.
   // Measured, whole tiles / 4 and 256 / 2 and 128 / 4 and 128 / 8 and 128 (one B200,
   // 21 pairs): 1024-pixel tiles of nside 64, 100 steps: 172 / 123 / 123 / 129 / 130 us;
   // 4096 of nside 128, 60 steps: 311 / 210 / 206 / 210 / 262; 16384 of nside 256, 60 steps:
@@ -899,9 +912,10 @@ int stage1_plan(const vb_sky* sky, const vb_baselines* bl, const vb_stage1_opts*
   // 20 steps without culling, nside 64: 116 us whole, 79 at 256 pixels, 69 at 128.
   if (o->chunk_pix == 0 && chunk == q.cull_tile) {
     q.whole_chunk = (int)chunk;
+    const bool few = coarse && (q.cull == VB_CULL_EXACT || (q.cull == VB_CULL_NONE && q.blockage));
     for (;;) {
       const int64_t have = ceil_div(q.npix, chunk) * q.n_btile;
-      if (!(chunk > 256 ? have < 4 * (int64_t)capacity : chunk > 128 && have < capacity)) break;
+      if (!(chunk > 256 ? have < (few ? 2 : 4) * (int64_t)capacity : chunk > 128 && have < capacity)) break;
       chunk /= 2;
     }
   }

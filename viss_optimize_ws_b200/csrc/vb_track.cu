@@ -597,7 +597,8 @@ __device__ __forceinline__ float4 pixel_at(const TrackArgs& a, int64_t p0, int n
 // lane's block, p0, np, cen its pixels and centre) into the warp's shared-memory
 // slots, scaled by their coefficients.  Eight lanes a block: the transposed
 // reduction of 2 J values then costs 7/8 N shuffles for four blocks instead of
-// 31/32 N for each (a quarter of a 64-pixel block's time, 8 % of a 256-pixel one).  With q = 2 kappa eta / (2 pi r) the generating function
+// 31/32 N for each (a quarter of a 64-pixel block's time, 8 % of a 256-pixel one).
+// With q = 2 kappa eta / (2 pi r) the generating function
 // e^{i (a tau + a^2 q / 2)} = sum_n (i a)^n g_n / n! has
 //   g_n = tau g_{n-1} - i (n - 1) q g_{n-2},
 // so that the curve costs five operations a power and the moments of z g_n
