@@ -3,12 +3,14 @@
 
 The pairs move along tracks of one direction at many speeds, so that every polynomial is
 met at the ends of its range.  Stage 1: the source is the pixel that lies farthest along the
-tracks from its block's centre; stage 2: the visibility is the last of a cluster.
+tracks (across them where they are noisy) from its block's centre; stage 2: the
+visibility is the last of a cluster.
 
 Tolerance for |exp(i phi)|: half a step of the 2^-23-turn phase grid 3.7e-7, the angle in
 float32 2.4e-7 and its fl(2 pi) 1.7e-7, the SFU's sine and cosine 6e-7, polynomials
-6e-7 and their float sums 5e-7 (powers up to 2.5^n / n!), 2.5e-6 in all; the
-per-term kernel's own bound, with three roundings of the phase, is 2.1e-6.  Stage 2:
+6e-7 and their float sums 5e-7 (powers up to 2.5^n / n!; 8e-7 and 1e-7 where residuals
+lead), 2.5e-6 in all; the per-term kernel's own bound, with three roundings of the
+phase, is 2.1e-6.  Stage 2:
 polynomials 1.5e-7 and their float sums 2e-7, 1.8e-6 in all.
 """
 from __future__ import annotations
@@ -23,14 +25,16 @@ pytestmark = pytest.mark.gpu
 TOL = 2.5e-6
 
 
-def tracks(vb, steps, speeds, axis, across, bend):
-    """Signed baselines of len(speeds) pairs: straight tracks with a bend of `bend` radians over 128 steps."""
+def tracks(vb, steps, speeds, axis, across, bend, noise=0.0):
+    """Signed baselines of len(speeds) pairs: straight tracks with a bend of `bend` radians over 128 steps, off
+    them by up to `noise` wavelengths (the first pair by little, the last by that)."""
     n = len(speeds)
     k = np.arange(steps)[:, None] - 0.5 * steps
     s = np.asarray(speeds)[None, :] * k
     c = s * (bend / 128) * k * 0.5
     start = np.stack([np.linspace(-300, 250, n), np.linspace(200, 330, n), np.linspace(30, -90, n)], 1)
     u = start[None] + s[:, :, None] * axis + c[:, :, None] * across
+    u = u + np.random.default_rng(8).uniform(-1, 1, u.shape) * (noise * np.linspace(0.02, 1, n))[None, :, None]
     full = np.concatenate([-u, u], 1).reshape(-1, 3).astype(np.float32)
     bl = vb.Baselines(n_full=full.shape[0], nbl=n)
     d = {key: dev(np.ascontiguousarray(full[:, i])) for i, key in enumerate("uvw")}
@@ -39,8 +43,9 @@ def tracks(vb, steps, speeds, axis, across, bend):
     return bl, d
 
 
-@pytest.mark.parametrize("nside,bend", [(512, 0.0), (512, 0.05), (512, 0.2), (256, 0.4), (128, 0.05)])
-def test_one_source(vb, gpu, nside, bend):
+@pytest.mark.parametrize("nside,bend,noise,fastest", [(512, 0.0, 0, 3.0), (512, 0.05, 0, 3.0), (512, 0.2, 0, 3.0), (256, 0.4, 0, 3.0),
+                                                      (128, 0.05, 0, 3.0), (512, 0.02, 0.008, 0.04), (512, 0.02, 0.005, 0.4)])
+def test_one_source(vb, gpu, nside, bend, noise, fastest):
     npix = min(12 * nside * nside, 1 << 20)
     (dl, dm, dn), lmn = geometry(nside)
     s = np.stack([a[:npix] for a in lmn], 1).astype(np.float64)
@@ -50,8 +55,10 @@ def test_one_source(vb, gpu, nside, bend):
         for p in np.argsort(-(t * t).sum(1))[:6:3]:
             axis = t[p] / np.linalg.norm(t[p])
             across = np.cross(s[p], axis)
+            if noise:                     # the source lies across the tracks: the residuals count
+                axis, across = across, axis
             steps = 128 * -(-(6_100_000_000 // (npix * 56)) // 128)
-            bl, keep = tracks(vb, max(steps, 256), np.geomspace(0.02, 3.0, 56), axis, across, bend)
+            bl, keep = tracks(vb, max(steps, 256), np.geomspace(0.02, fastest, 56), axis, across, bend, noise)
             B = np.zeros(npix, np.float32)
             B[p] = 1.0
             dB = dev(B)

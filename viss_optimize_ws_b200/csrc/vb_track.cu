@@ -13,8 +13,8 @@
 // in a for the curve's factor, times the residuals to first order.  The warp
 // forms the polynomial's moments over the pixels once per (group, block), then
 // every baseline of the group evaluates it.  A group is taken only where any
-// single term is off by at most 6e-7 (vb_series.h: 1e-7 for the polynomial, the
-// rest for the residuals, at a block's edge and a group's end); the phase of z_p is
+// single term is off by at most 6e-7 to 8e-7 (vb_series.h: 1e-7 for the polynomial,
+// the rest for the residuals, at a block's edge and a group's end); the phase of z_p is
 // rounded once here and three times in the per-term kernel, 3.7e-7 against 1.1e-6,
 // so that a term is no further off than there.  Measured on skies of one source,
 // largest and rms error of a term: 1.5e-6 and 3.4e-7, per-term kernel 1.5e-6 and
