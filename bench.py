@@ -278,12 +278,16 @@ def traffic_from_profiles(kernel: str, workload: str) -> float | None:
     return None
 
 
-def factors(terms: float, steps: float, cfg, line: float, least_steps: int) -> bool:
-    """Whether the library may sum several steps of a pair together on this workload
-    (from `line` terms and `least_steps` steps, FP32 sum with FP64 phase; it decides
-    on the device): its term counters then count what a direct sum evaluates."""
+def may_factor(p, r: dict) -> tuple[bool, bool]:
+    """Whether the library may sum several steps of a pair together in stage 1 and stage 2
+    of this workload (FP32 sum with FP64 phase: from 6e9 terms and 96 steps, from 3e10
+    pairs and 64 steps a segment; it decides on the device): its term counters then
+    count what a direct sum evaluates."""
     import viss_optimize_ws_b200 as vb
-    return cfg.precision == vb.PREC_FP32_FP64PH and terms >= line and steps >= least_steps
+    if p.cfg.precision != vb.PREC_FP32_FP64PH:
+        return False, False
+    terms, steps = r["stage1_terms"], p.n_half / p.nbl
+    return terms >= 6e9 and steps >= 96, (1 if p.cfg.mirror else 2) * terms >= 3e10 and steps >= 64 * p.nseg
 
 
 def stage_rate(kernel: str, terms: int, kernel_ms: float, stage_ms: float, peak: float, factored: bool) -> dict:
@@ -559,13 +563,16 @@ def run_config_report(args) -> None:
         r = t["report"]
         ev = err_report(p.get("V_half"), V64, True)
         ec = err_report(p.get("C"), C64, False)
+        # the direct sum's terms over the kernels' time, of the SFU peak: a fraction of it where nothing is factored
+        ratio = [(r[f"s{k}_counters"][0] + r[f"s{k}_counters"][1]) / (t[f"t_s{k}_kernel_ms"] * 1e-3) / 1e9 / peak for k in (1, 2)]
+        frac = [None if f else x for f, x in zip(may_factor(p, r), ratio)]
         out["mixed"][prec] = {
             "ms_per_step": t["ms_per_step"], "gterm_s": t["gterm_s"], "speedup_vs_fp64": t64["ms_per_step"] / t["ms_per_step"],
             "stage1_kernel_ms": t["t_s1_kernel_ms"], "stage2_kernel_ms": t["t_s2_kernel_ms"],
             "stage1_eval_terms": int(r["s1_counters"][0] + r["s1_counters"][1]),
             "stage2_eval_terms": int(r["s2_counters"][0] + r["s2_counters"][1]),
-            "stage1_sfu_frac": (r["s1_counters"][0] + r["s1_counters"][1]) / (t["t_s1_kernel_ms"] * 1e-3) / 1e9 / peak,
-            "stage2_sfu_frac": (r["s2_counters"][0] + r["s2_counters"][1]) / (t["t_s2_kernel_ms"] * 1e-3) / 1e9 / peak,
+            "stage1_sfu_frac": frac[0], "stage2_sfu_frac": frac[1],
+            "stage1_direct_sum_ratio": ratio[0], "stage2_direct_sum_ratio": ratio[1],
             "err_V": ev, "err_C": ec, "W_equal_fp64": bool(np.array_equal(p.get("W"), W64)),
             "error_flags": r["error_flags"], "autotune": tune}
         if prec == "fp32_fp64phase" and n == 5:
@@ -856,9 +863,7 @@ def main() -> None:
 
     # rate of each stage, of the SFU's where the stage is a direct sum
     s1c, s2c = r["s1_counters"], r["s2_counters"]
-    steps_day = p.n_half / p.nbl
-    f1 = factors(r["stage1_terms"], steps_day, p.cfg, 6e9, 96)
-    f2 = factors((1 if p.cfg.mirror else 2) * r["stage1_terms"], steps_day / p.nseg, p.cfg, 3e10, 64)
+    f1, f2 = may_factor(p, r)
     peak_terms = sfu.value / 1e9          # G sincos pairs per second
     k1_ms = t_k1 / args.steps
     roofline = stage_rate("k_stage1 + k_track_sum" if f1 else "k_stage1", int(s1c[0] + s1c[1]), k1_ms, t_s1 / args.steps, peak_terms, f1)

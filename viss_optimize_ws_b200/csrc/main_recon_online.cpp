@@ -300,7 +300,7 @@ int main(int argc, char** argv) {
   cfg.device = 0;
 
   // --report_json: the SFU (sin + cos) rate of this GPU, measured once, is the
-  // denominator of the per-stage roofline fractions of each day
+  // denominator of the per-stage rates of each day
   double sfu_pairs = 0.0;
   if (!report_json.empty()) {
     double f32 = 0, f64 = 0, clk = 0;
@@ -586,7 +586,8 @@ int main(int argc, char** argv) {
          << rep.s1_counters[1] << ", " << rep.s1_counters[2] << ", " << rep.s1_counters[3]
          << "], \"s2_counters\": [" << rep.s2_counters[0] << ", " << rep.s2_counters[1] << ", "
          << rep.s2_counters[2] << ", " << rep.s2_counters[3] << "]";
-    // evaluated terms (visible-fast + masked) per second over the kernel time, against the SFU rate
+    // terms that a direct sum evaluates (visible-fast + masked) per second over the kernel time, against the SFU
+    // rate: a roofline fraction where no steps are summed together, a ratio that may pass 1 where some are
     auto frac = [&](const unsigned long long* c, double ms) {
       return (sfu_pairs > 0 && ms > 0) ? (double)(c[0] + c[1]) / (ms * 1e-3) / sfu_pairs : 0.0;
     };
