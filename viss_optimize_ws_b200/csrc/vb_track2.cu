@@ -13,8 +13,8 @@
 // per (cluster, block), a lane per group, and every pixel evaluates it.  The
 // phase of a pixel's factor is rounded once to the 2^-23-turn grid, where
 // k_recon_rec rounds twice, 3.7e-7 against 7.5e-7, so that a term is no further off
-// than there (1.5 % of the kernel's time).  Measured with one visibility, largest and
-// rms error of a term: 1.1e-6 and 2.4e-7, k_recon_rec 1.2e-6 and 2.7e-7.  Clusters
+// than there.  Measured with one visibility, largest and rms error of a term: 1.1e-6
+// and 2.4e-7, k_recon_rec 1.2e-6 and 2.7e-7.  Clusters
 // that no polynomial fits and groups outside clusters stay on k_recon_rec.
 //
 // Bound: FP32 issue (per cluster and 1024 pixels: 4 x (32 groups' classes, FP64
@@ -537,8 +537,7 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
           lp[q] = fma((double)fa, (double)nf[q], (double)lf[q]);
           mp[q] = fma((double)fb, (double)nf[q], (double)mf[q]);
         }
-        auto angle = [&](double A, double B, int q, bool odd, float& s, float& c) {
-          const double t = fma(A, lp[q], B * mp[q]) + kMagic;   // one rounding to the grid
+        auto angle = [&](double t, bool odd, float& s, float& c) {
           const unsigned kb = ((unsigned)__double2loint(t) & 0x7FFFFFu) ^ (odd ? 0x4B400000u : 0x4B000000u);
           __sincosf(__fmaf_rn(__uint_as_float(kb), kAngScale, -kTwoPiF), &s, &c);
         };
@@ -561,7 +560,7 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
             for (int q = 0; q < G2_PPT; ++q) {
               // odd clusters half a turn on with the opposite sign (the SFU's mean error cancels)
               float s, c;
-              angle(st.A, st.B, q, k & 1, s, c);
+              angle(fma(st.A, lp[q], st.B * mp[q]) + kMagic, k & 1, s, c);   // one rounding to the grid
               const float v = fmaf(h[q].x, c, -h[q].y * s);
               acc[q] += (k & 1) ? -v : v;
               totW[q] += (unsigned)nv;
@@ -580,7 +579,7 @@ __global__ void __launch_bounds__(G2_THREADS, 2) k_recon_track(const __grid_cons
               const bool in = !a.blockage || (occ_dot(lf[q], mf[q], nf[q], p1.x, p1.y, p1.z, p1.w) >= cp1 &&
                                               occ_dot(lf[q], mf[q], nf[q], p2.x, p2.y, p2.z, p2.w) >= cp2);
               float s, c;
-              angle(ga, gb, q, src & 1, s, c);
+              angle(fma(ga, lp[q], fma(gb, mp[q], kMagic)), src & 1, s, c);   // a term of its own, as in k_recon_rec
               const float vv = fmaf(vx, c, -vy * s);
               if (in) {
                 acc[q] += (src & 1) ? -vv : vv;
