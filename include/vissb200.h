@@ -326,7 +326,9 @@ size_t vb_stage2_workspace_bytes(int n_half_total, int nseg, int64_t npix,
  * stable (key, index) sort, run-length groups, representatives
  * (idx_sorted[s0 + (L>>1)]), then one reconstruction launch over
  * (pixel block x group chunk) and the normalisation C = sum C / sum W.
- * seg_t0/seg_tlen: device int arrays (steps, relative to the baselines given);
+ * seg_t0/seg_tlen: device int arrays (steps, relative to the baselines given; a step
+ * belongs to the last entry that begins at or before it, and the plane fit of an entry
+ * takes those of its steps that the baselines hold);
  * V_half: phase-corrected float2 of every half-baseline (from
  * vb_phase_correct_expand).  Outputs C (npix float), W (npix uint32,
  * nullable), seg_params (device, nseg entries, nullable) and

@@ -1,5 +1,5 @@
 """Stage 2 with clusters of uv groups (vb_track2.cu) on segment tables whose ranges
-overlap, repeat a start or are out of order: what the FP64 build gives, which sums
+overlap, repeat a start, are out of order or leave the day: what the FP64 build gives, which sums
 every group by itself, the same bits on every call, and each group once (W).
 
 Tolerance: as in test_gpu_clusters.py (4e-7 rms a term, 1.5e-6 for the largest).
@@ -36,6 +36,8 @@ def per_group(vb, sky, bl, dV, t0, tl, lam):
     ([0, 0, 150], [300, 500, 350], True),        # the first entry has no step of its own
     ([250, 0], [250, 250], True),                # out of order
     ([100, 100, 350], [120, 60, 150], True),     # steps before the first entry and between two
+    ([0, 300], [300, 400], True),                # past the day's end
+    ([-50, 250], [300, 250], True),              # from before its start
 ])
 def test_clusters_on_any_segment_table(vb, gpu, t0, tl, clusters):
     sky, bl, V, keep = setup(vb, 512, 2200001, 300.0, 500, 1)

@@ -90,11 +90,13 @@ __device__ __forceinline__ dd dd_shfl_xor(dd a, int m) {
 __global__ void __launch_bounds__(kFitThreads) k_seg_fit(const float* __restrict__ u, const float* __restrict__ v,
                                                  const float* __restrict__ w, int nbl, const int* __restrict__ seg_t0,
                                                  const int* __restrict__ seg_tlen, float bl_max, float lambda,
-                                                 int grid_res, int mirror, vb_seg_params* __restrict__ out) {
+                                                 int grid_res, int mirror, int steps, vb_seg_params* __restrict__ out) {
   __shared__ dd red[5][kFitThreads / 32];
   const int s = blockIdx.x;
-  const int i0 = 2 * nbl * seg_t0[s];
-  const int n = 2 * nbl * seg_tlen[s];
+  // the steps that the baselines hold: a table may run past them
+  const int t0 = max(0, seg_t0[s]), t1 = (int)min((int64_t)steps, (int64_t)seg_t0[s] + seg_tlen[s]);
+  const int i0 = 2 * nbl * t0;
+  const int n = t1 > t0 ? 2 * nbl * (t1 - t0) : 0;
   dd a[5];
   for (int k = 0; k < 5; ++k) a[k] = {0.0, 0.0};
 #pragma unroll 2
@@ -1221,7 +1223,7 @@ int stage2_group(const vb_sky* sky, const vb_baselines* bl, int nseg, const int*
   if (g > sm_count() * 16) g = sm_count() * 16;
   // 1. per-segment fit
   k_seg_fit<<<nseg, kFitThreads, 0, st>>>(bl->u, bl->v, bl->w, nbl, seg_t0, seg_tlen, p.bl_max, p.lambda, p.grid_res,
-                                  p.mirror, x.sp);
+                                  p.mirror, p.n_half_total / nbl, x.sp);
   VB_LAUNCH_CHECK();
   if (n > 0) {
     // 2. keys
